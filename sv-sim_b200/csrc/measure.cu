@@ -26,16 +26,17 @@
 //                     guessed crossing, or no normal start);
 //   3. k_cdf_super    per superblock: the sum of its blocks' D_b when they share one
 //                     binade, else "no delta";
-//   4. k_cdf_chain    one warp walks the superblocks in order from S = 0: a delta
+//   4. k_cdf_chain    one CTA walks the superblocks in order from S = 0: a delta
 //                     applies when S is in its binade and stays there (checked on the
-//                     exact S), otherwise the warp descends to blocks and, where a
-//                     block's delta does not apply either, to chunks of 32 elements
-//                     (chunk_scan_exact);
+//                     exact S), otherwise the CTA descends to blocks and, where a
+//                     block's delta does not apply either, through the block's chunks
+//                     of 32 elements (walk_block);
 //   5. k_cdf_fill     the exact S at every block start of the superblocks the chain
 //                     did not descend into;
 //   6. k_sample_exact one warp per shot: binary search over the exact block starts,
-//                     then chunk_scan_exact through the block to the first index whose
-//                     inclusive S exceeds r.
+//                     then groups of 512 elements, their chunks and one chunk's exact sums
+//                     to the first index whose inclusive S exceeds r.
+// States of at most WALK_BLOCKS blocks skip passes 1-3 and 5: the chain walks every block.
 // Every step computes the reference's sequential values themselves, so equal inputs
 // give the reference's samples whatever the summation order of pass 1.
 #include "gate_math.cuh"
@@ -46,6 +47,9 @@ namespace {
 constexpr int BLOCK_AMPS = 1 << MEAS_BLOCK_BITS;   // 4096
 constexpr int CHUNKS = BLOCK_AMPS / 32;            // 128
 constexpr int SUPER_BLOCKS = 1 << MEAS_SUPER_BITS; // 64
+// Up to here walking every block (a few us each) is shorter than the five launches that
+// would spare the chain some of them; a state this small has a binade crossing in most.
+constexpr uint64_t WALK_BLOCKS = 4;
 constexpr uint64_t FRAC_MASK = (1ull << 52) - 1;
 constexpr uint64_t HIDDEN = 1ull << 52;
 constexpr uint64_t M_MAX = (1ull << 53) - 1;       // largest grid count inside one binade
@@ -170,37 +174,135 @@ __device__ __forceinline__ double chunk_scan_exact(double s_in, double p, int la
     return mine;
 }
 
+// The chain's CTA.  Its 16 warps share one block's probabilities in shared memory; one warp
+// alone walked a block in 48-190 us (128 dependent chunk loads and scans), and a state has
+// a walked block per binade that S crosses, 12 to 25 of them.
+constexpr int CHAIN_THREADS = 512;
+struct WalkSmem {
+    double p[BLOCK_AMPS];
+    uint64_t delta[CHUNKS];          // a chunk's grid units in the current binade
+    uint32_t ok[CHUNKS];             // no tie, NaN or inf among them
+};
+
+// S after block b, exactly, from s at its start; every thread of the CTA calls it with the
+// same s and receives the same result.  The chunks' grid units are summed for the current
+// binade by all warps at once; a warp-wide scan over the 128 chunks (four a lane, the same
+// in every warp) finds the first chunk that ties or leaves the binade, that chunk is added
+// element by element, and the sums are formed again only when the binade changed.
 template <typename T>
 __device__ double walk_block(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t b,
-                             double s, int lane)
+                             double s, WalkSmem& sm)
 {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t base = b * BLOCK_AMPS;
-    for (int c = 0; c < CHUNKS; c++) {
-        const uint64_t i0 = base + (uint64_t)c * 32;
-        if (i0 >= dim) break;
-        const double incl = chunk_scan_exact(s, prob_at<T>(sv, dim, i0 + lane), lane);
-        s = __shfl_sync(0xffffffffu, incl, 31);
+    const int chunks = dim - base < BLOCK_AMPS ? (int)((dim - base + 31) / 32) : CHUNKS;
+    __syncthreads();                         // the previous block's readers are done
+#pragma unroll
+    for (int k = 0; k < BLOCK_AMPS / CHAIN_THREADS; k++)
+        sm.p[tid + k * CHAIN_THREADS] = prob_at<T>(sv, dim, base + tid + k * CHAIN_THREADS);
+    uint32_t have = 0;                       // binade code sm.delta is formed for
+    int cur = 0;
+    while (cur < chunks) {
+        uint64_t m = 0;
+        const uint32_t code = binade_of(s, &m);
+        int f = cur;                         // chunk to add element by element
+        if (code != 0) {
+            if (code != have) {
+                __syncthreads();             // sm.p is written; readers of the old sums are done
+#pragma unroll
+                for (int k = 0; k < CHUNKS * 32 / CHAIN_THREADS; k++) {
+                    const int c = warp + k * (CHAIN_THREADS / 32);
+                    bool ok = true;
+                    const uint64_t d = warp_sum_u64(grid_units(sm.p[c * 32 + lane], code, &ok));
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (lane == 0) {
+                        sm.delta[c] = d;     // each unit is at most 2^53: no wrap
+                        sm.ok[c] = ok;
+                    }
+                }
+                __syncthreads();
+                have = code;
+            }
+            // inclusive sums of the chunks from cur on; a chunk with a tie ends the run.
+            // Sums are capped just above M_MAX so that 128 of them cannot wrap.
+            constexpr uint64_t OVER = 1ull << 54;
+            uint64_t v[4], run = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int c = lane * 4 + k;
+                const uint64_t d = (c < cur || c >= chunks) ? 0 : (sm.ok[c] && sm.delta[c] <= M_MAX ? sm.delta[c] : OVER);
+                run = run + d < OVER ? run + d : OVER;
+                v[k] = run;
+            }
+            uint64_t incl = run;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl = incl + y < OVER ? incl + y : OVER;
+            }
+            const uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
+            const uint64_t excl = lane ? before : 0;
+            int bad = 4;                     // first of this lane's chunks that does not fit
+#pragma unroll
+            for (int k = 3; k >= 0; k--)
+                if (excl + v[k] > M_MAX - m) bad = k;
+            const unsigned who = __ballot_sync(0xffffffffu, bad < 4);
+            uint64_t pre = 0;                // grid units before chunk f
+            if (who) {
+                const int l = __ffs(who) - 1;
+                const uint64_t mine = excl + (bad == 0 || bad == 4 ? 0 : v[bad - 1]);
+                pre = __shfl_sync(0xffffffffu, mine, l);
+                f = l * 4 + __shfl_sync(0xffffffffu, bad, l);
+            } else {
+                pre = __shfl_sync(0xffffffffu, incl, 31);
+                f = chunks;
+            }
+            s = from_grid(code, m + pre);
+            if (f >= chunks) break;
+        } else {
+            if (s != s) break;               // NaN stays NaN
+            if (have == 0) {
+                __syncthreads();
+                have = ~0u;                  // sm.p is written; no sums formed
+            }
+            if (s == 0.0 && __all_sync(0xffffffffu, sm.p[f * 32 + lane] == 0.0)) {
+                cur = f + 1;
+                continue;
+            }
+        }
+        double x = s;
+#pragma unroll
+        for (int k = 0; k < 32; k++) x = __dadd_rn(x, sm.p[f * 32 + k]);
+        s = x;
+        cur = f + 1;
     }
     return s;
 }
 
+// One CTA per block of 4,096 amplitudes, 16 loads in flight a thread: HBM-bound for large
+// states; with one warp per block a 2^16-amplitude state took 75 us on 16 warps.
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_block_sums(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t nblocks,
              double* __restrict__ out)
 {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t b = warp; b < nblocks; b += nwarps) {
-        const uint64_t base = b * BLOCK_AMPS;
-        double acc = 0.0;
-        for (int c = 0; c < CHUNKS; c++) {
-            const uint64_t i0 = base + (uint64_t)c * 32;
-            if (i0 >= dim) break;
-            acc += warp_sum(prob_at<T>(sv, dim, i0 + lane));
+    __shared__ double red[8];
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (uint64_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
+        const uint64_t base = b * BLOCK_AMPS + tid;
+        double q[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 16; k++) q[k & 3] += prob_at<T>(sv, dim, base + k * 256);
+        const double acc = warp_sum((q[0] + q[1]) + (q[2] + q[3]));
+        if (lane == 0) red[tid >> 5] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            double t = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) t += red[w];
+            out[b] = t;
         }
-        if (lane == 0) out[b] = acc;
+        __syncthreads();
     }
 }
 
@@ -246,7 +348,7 @@ k_scan_single(const double* __restrict__ in, uint64_t count, double* __restrict_
     if (t == 1023) out[count] = wsum[31] + incl;
 }
 
-// Pass 2: one warp per block.  The binade guess is that of the approximate prefix at
+// Pass 2: one CTA per block.  The binade guess is that of the approximate prefix at
 // the block's start; a block whose approximate end lies in another binade is left
 // without a delta (the chain adds it element by element).
 template <typename T>
@@ -254,35 +356,41 @@ __global__ void __launch_bounds__(256)
 k_cdf_blocks(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t nblocks,
              const double* __restrict__ approx, uint64_t* __restrict__ entry)
 {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t b = warp; b < nblocks; b += nwarps) {
+    __shared__ uint64_t red[8];
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (uint64_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
         uint64_t m0, m1;
         const uint32_t c0 = binade_of(approx[b], &m0);
         const uint32_t c1 = binade_of(approx[b + 1], &m1);
         const uint32_t code = (c0 != 0 && c0 == c1) ? c0 : 0;
-        const uint64_t base = b * BLOCK_AMPS;
+        const uint64_t base = b * BLOCK_AMPS + tid;
+        double p[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) p[k] = prob_at<T>(sv, dim, base + k * 256);
         uint64_t acc = 0;
         bool ok = true, nonzero = false, nan_free = true;
-        for (int c = 0; c < CHUNKS; c++) {
-            const uint64_t i0 = base + (uint64_t)c * 32;
-            if (i0 >= dim) break;
-            const double p = prob_at<T>(sv, dim, i0 + lane);
-            nonzero |= (p != 0.0);
-            nan_free &= (p == p);
-            if (code != 0) acc += grid_units(p, code, &ok);
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            nonzero |= (p[k] != 0.0);
+            nan_free &= (p[k] == p[k]);
+            if (code != 0) acc += grid_units(p[k], code, &ok);
         }
-        nonzero = __any_sync(0xffffffffu, nonzero);
-        nan_free = __all_sync(0xffffffffu, nan_free);
-        ok = __all_sync(0xffffffffu, ok);
-        acc = warp_sum_u64(acc);               // < 4096 * 2^52: no wrap
-        if (lane == 0) {
+        acc = warp_sum_u64(acc);               // 4096 terms of at most 2^52: no wrap
+        if (lane == 0) red[tid >> 5] = acc;
+        // the barriers below also order red[] before its readers and the next block's writers
+        nonzero = __syncthreads_or(nonzero);
+        nan_free = __syncthreads_and(nan_free);
+        ok = __syncthreads_and(ok);
+        if (tid == 0) {
+            acc = 0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) acc += red[w];
             uint64_t w = pack_entry(nan_free ? 1 : 0, CODE_NONE);
             if (!nonzero) w = pack_entry(0, CODE_ZERO);
             else if (code != 0 && ok && acc < HIDDEN) w = pack_entry(acc, code);
             entry[b] = w;
         }
+        __syncthreads();
     }
 }
 
@@ -323,49 +431,97 @@ __device__ __forceinline__ bool stuck(double s, uint64_t w)
     return isinf(s) && (entry_code(w) != CODE_NONE || entry_delta(w) == 1);
 }
 
-// Pass 4: one warp.  Entries are read 32 at a time (one per lane) and broadcast, so
-// the chain waits on memory once per 32 superblocks or blocks.  desc[s] = 1 marks a
-// superblock whose block starts the chain wrote itself.
+// S over 32 consecutive superblocks (or blocks) at once: lane l holds entry w of the l-th of
+// them (cnt in all).  When every entry is zero or a delta of S's binade and S stays in the
+// binade, *s is advanced past all of them and *excl receives S at this lane's start.
+__device__ __forceinline__ bool advance_32(double* s, uint64_t w, uint64_t cnt, int lane, double* excl)
+{
+    uint64_t m;
+    const uint32_t code = binade_of(*s, &m);
+    if (code == 0) return false;
+    const uint32_t c = entry_code(w);
+    const bool in = (uint64_t)lane < cnt;
+    if (!__all_sync(0xffffffffu, !in || c == CODE_ZERO || c == code)) return false;
+    const uint64_t d = (in && c == code) ? entry_delta(w) : 0;     // each < 2^52
+    uint64_t incl = d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const uint64_t total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total > M_MAX - m) return false;
+    *excl = from_grid(code, m + (incl - d));
+    *s = from_grid(code, m + total);
+    return true;
+}
+
+// Pass 4: one CTA; every warp follows the same chain (S and the entries are the same in
+// all), warp 0 writes it down, and all of them share the work of a walked block.  Entries
+// are read 32 at a time (one per lane) and, where they are all deltas of S's binade, added
+// by one scan; else one by one.  desc[s] = 1 marks a superblock whose block starts the
+// chain wrote itself.  entry == nullptr: no deltas, every block is walked.
 template <typename T>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(CHAIN_THREADS)
 k_cdf_chain(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t nblocks,
             uint64_t nsuper, const uint64_t* __restrict__ entry, const uint64_t* __restrict__ sentry,
             double* __restrict__ start, double* __restrict__ sstart, uint32_t* __restrict__ desc)
 {
-    const int lane = threadIdx.x;
-    double s_val = 0.0;
+    __shared__ WalkSmem sm;
+    const int lane = threadIdx.x & 31;
+    const bool writer = threadIdx.x == 0, wwarp = threadIdx.x < 32;
+    double s_val = 0.0, at;
+    if (!entry) {
+        for (uint64_t b = 0; b < nblocks; b++) {
+            if (writer) start[b] = s_val;
+            s_val = walk_block<T>(sv, dim, b, s_val, sm);
+        }
+        if (writer) start[nblocks] = s_val;
+        return;
+    }
     for (uint64_t g = 0; g < nsuper; g += 32) {
         const uint64_t mine = g + lane < nsuper ? sentry[g + lane] : 0;
         const uint64_t cnt = nsuper - g < 32 ? nsuper - g : 32;
+        if (advance_32(&s_val, mine, cnt, lane, &at)) {
+            if (wwarp && (uint64_t)lane < cnt) {
+                sstart[g + lane] = at;
+                desc[g + lane] = 0;
+            }
+            continue;
+        }
         for (uint64_t k = 0; k < cnt; k++) {
             const uint64_t sidx = g + k;
             const uint64_t w = __shfl_sync(0xffffffffu, mine, (int)k);
-            if (lane == 0) sstart[sidx] = s_val;
+            if (writer) sstart[sidx] = s_val;
             const uint32_t code = entry_code(w);
             if (code == CODE_ZERO || stuck(s_val, w) ||
                 (code != CODE_NONE && advance(&s_val, code, entry_delta(w)))) {
-                if (lane == 0) desc[sidx] = 0;
+                if (writer) desc[sidx] = 0;
                 continue;
             }
-            if (lane == 0) desc[sidx] = 1;
+            if (writer) desc[sidx] = 1;
             const uint64_t b0 = sidx * SUPER_BLOCKS;
             const uint64_t b1 = b0 + SUPER_BLOCKS < nblocks ? b0 + SUPER_BLOCKS : nblocks;
             for (uint64_t h = b0; h < b1; h += 32) {
                 const uint64_t bm = h + lane < b1 ? entry[h + lane] : 0;
                 const uint64_t bc = b1 - h < 32 ? b1 - h : 32;
+                if (advance_32(&s_val, bm, bc, lane, &at)) {
+                    if (wwarp && (uint64_t)lane < bc) start[h + lane] = at;
+                    continue;
+                }
                 for (uint64_t j = 0; j < bc; j++) {
                     const uint64_t b = h + j;
                     const uint64_t wb = __shfl_sync(0xffffffffu, bm, (int)j);
-                    if (lane == 0) start[b] = s_val;
+                    if (writer) start[b] = s_val;
                     const uint32_t cb = entry_code(wb);
                     if (cb == CODE_ZERO || stuck(s_val, wb)) continue;
                     if (cb != CODE_NONE && advance(&s_val, cb, entry_delta(wb))) continue;
-                    s_val = walk_block<T>(sv, dim, b, s_val, lane);
+                    s_val = walk_block<T>(sv, dim, b, s_val, sm);
                 }
             }
         }
     }
-    if (lane == 0) {
+    if (writer) {
         start[nblocks] = s_val;
         sstart[nsuper] = s_val;
     }
@@ -417,7 +573,49 @@ k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uin
         const uint64_t base = lo * BLOCK_AMPS;
         double s = start[lo];
         result = ~0ull;                  // replaced below: start[lo+1] > r is met inside the block
-        for (int c = 0; c < CHUNKS; c++) {
+        int c0 = 0, c1 = CHUNKS;         // chunks still to look through one by one
+        // groups of 16 chunks, their 16 loads a lane in flight together (one chunk at a
+        // time, a shot waited for up to 128 loads in turn: 95 us for 1,024 shots): a group
+        // without ties that stays in S's binade and ends at or below r is stepped over, and
+        // in the first that ends above r its chunks' sums are looked through the same way
+        for (int g = 0; g < CHUNKS; g += 16) {
+            uint64_t m;
+            const uint32_t code = binade_of(s, &m);
+            c0 = g;
+            if (code == 0) break;
+            bool ok = true;
+            uint64_t d[16], sum = 0;
+#pragma unroll
+            for (int c = 0; c < 16; c++)
+                d[c] = grid_units(prob_at<T>(sv, dim, base + (uint64_t)(g + c) * 32 + lane), code, &ok);
+#pragma unroll
+            for (int c = 0; c < 16; c++) sum += d[c];
+            sum = warp_sum_u64(sum);     // 512 terms of at most 2^53: no wrap
+            if (!__all_sync(0xffffffffu, ok) || sum > M_MAX - m) break;
+            const double end = from_grid(code, m + sum);
+            if (end <= r) {
+                s = end;
+                c0 = CHUNKS;
+                continue;
+            }
+            uint64_t pre = 0;            // units of the chunks that end at or below r
+            int f = 0;
+            bool open = true;
+#pragma unroll
+            for (int c = 0; c < 16; c++) {
+                const uint64_t t = warp_sum_u64(d[c]);
+                open = open && from_grid(code, m + pre + t) <= r;
+                if (open) {
+                    pre += t;
+                    f = c + 1;
+                }
+            }
+            s = from_grid(code, m + pre);
+            c0 = g + f;                  // f < 16: the group ends above r
+            c1 = c0 + 1;
+            break;
+        }
+        for (int c = c0; c < c1; c++) {
             const uint64_t i0 = base + (uint64_t)c * 32;
             if (i0 >= dim) break;
             const double incl = chunk_scan_exact(s, prob_at<T>(sv, dim, i0 + lane), lane);
@@ -566,17 +764,20 @@ cudaError_t measure_device(const void* state, int n, const double* d_uniforms, u
     uint64_t* sentry = reinterpret_cast<uint64_t*>(base + L.off_sentry);
     double* sstart = base + L.off_sstart;
     uint32_t* desc = reinterpret_cast<uint32_t*>(base + L.off_desc);
-    // 1. approximate block sums (into the entry array) and their prefix (into start)
-    unsigned blocks = (unsigned)((L.nblocks * 32 + 255) / 256);
-    if (blocks > 148u * 16) blocks = 148u * 16;
-    k_block_sums<T><<<blocks, 256, 0, s>>>(sv, dim, L.nblocks, base + L.off_entry);
-    k_scan_single<<<1, 1024, 0, s>>>(base + L.off_entry, L.nblocks, start);
-    // 2-5. exact block starts
-    k_cdf_blocks<T><<<blocks, 256, 0, s>>>(sv, dim, L.nblocks, start, entry);
-    const unsigned sb = (unsigned)((L.nsuper + 255) / 256);
-    k_cdf_super<<<sb, 256, 0, s>>>(entry, L.nblocks, L.nsuper, sentry);
-    k_cdf_chain<T><<<1, 32, 0, s>>>(sv, dim, L.nblocks, L.nsuper, entry, sentry, start, sstart, desc);
-    k_cdf_fill<<<sb, 256, 0, s>>>(entry, L.nblocks, L.nsuper, sstart, desc, start);
+    const unsigned blocks = (unsigned)(L.nblocks < 148u * 16 ? L.nblocks : 148u * 16);
+    if (L.nblocks <= WALK_BLOCKS) {
+        k_cdf_chain<T><<<1, CHAIN_THREADS, 0, s>>>(sv, dim, L.nblocks, L.nsuper, nullptr, nullptr, start, sstart, desc);
+    } else {
+        // 1. approximate block sums (into the entry array) and their prefix (into start)
+        k_block_sums<T><<<blocks, 256, 0, s>>>(sv, dim, L.nblocks, base + L.off_entry);
+        k_scan_single<<<1, 1024, 0, s>>>(base + L.off_entry, L.nblocks, start);
+        // 2-5. exact block starts
+        k_cdf_blocks<T><<<blocks, 256, 0, s>>>(sv, dim, L.nblocks, start, entry);
+        const unsigned sb = (unsigned)((L.nsuper + 255) / 256);
+        k_cdf_super<<<sb, 256, 0, s>>>(entry, L.nblocks, L.nsuper, sentry);
+        k_cdf_chain<T><<<1, CHAIN_THREADS, 0, s>>>(sv, dim, L.nblocks, L.nsuper, entry, sentry, start, sstart, desc);
+        k_cdf_fill<<<sb, 256, 0, s>>>(entry, L.nblocks, L.nsuper, sstart, desc, start);
+    }
     // 6. samples
     if (shots > 0) {
         const unsigned sblocks = (unsigned)(((uint64_t)shots * 32 + 255) / 256);
@@ -596,8 +797,7 @@ cudaError_t norm2_device(const void* state, int n, double* d_total, MeasureScrat
     const MeasureLayout L = measure_layout(n);
     if (!scr.cdf || scr.cap_doubles < L.doubles) return cudaErrorInvalidValue;
     double* base = scr.cdf;
-    unsigned blocks = (unsigned)((L.nblocks * 32 + 255) / 256);
-    if (blocks > 148u * 16) blocks = 148u * 16;
+    const unsigned blocks = (unsigned)(L.nblocks < 148u * 16 ? L.nblocks : 148u * 16);
     k_block_sums<T><<<blocks, 256, 0, s>>>(static_cast<const V*>(state), 1ull << n, L.nblocks, base + L.off_entry);
     k_scan_single<<<1, 1024, 0, s>>>(base + L.off_entry, L.nblocks, base + L.off_start);
     cudaError_t e = cudaMemcpyAsync(d_total, base + L.off_start + L.nblocks, sizeof(double),

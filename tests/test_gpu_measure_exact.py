@@ -148,3 +148,21 @@ def test_small_states(oracle):
         h.run()
         h.sync()
         check_state(oracle, h, n, np.random.default_rng(n), count=min(300, 1 << n))
+
+
+@pytest.mark.parametrize("n", [13, 14, 15, 18, 19])
+@pytest.mark.parametrize("maker", [None, tie_state, tiny_then_large_state])
+def test_edges_around_the_walked_sizes(oracle, n, maker):
+    """States of 4 blocks (n = 14) have every block walked, from 5 blocks on (n = 15) the
+    block deltas come first, from 65 blocks on (n = 19) a second superblock: exact on both
+    sides of each line, from random states and with ties and crossings in every block."""
+    nat = native()
+    rng = np.random.default_rng(1000 + n)
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    if maker is None:
+        st = rng.standard_normal((2, 1 << n))
+        st /= np.sqrt((st ** 2).sum())
+    else:
+        st = maker(n, rng)
+    h.set_state(st[0], st[1])
+    check_state(oracle, h, n, rng)
