@@ -355,15 +355,18 @@ def run_ours(args):
     achieved = per_launch_bytes / launch_s / 1e9
     peak, peak_kind = peaks()
     traffic = None
+    # without tensor-core blocks the pair engine runs its butterfly form
+    butterflies = args.engine == "pairs" and int(info.n_blocks) == 0
     tfile = os.path.join(ROOT, "profiles", "pairs_fp64_traffic.txt" if args.engine == "pairs"
                          else "staged_fp64_traffic.txt")
-    if os.path.exists(tfile):
+    if os.path.exists(tfile) and not butterflies:
         for ln in open(tfile):
             if ln.startswith("bytes_per_launch_n30"):
                 traffic = float(ln.split("=")[1])
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
-                "kernel": ("k_pairs (FP64 mma.sync two-qubit blocks)" if args.engine == "pairs"
+                "kernel": ("k_bfly (FP64 gates as butterflies in registers)" if butterflies
+                           else "k_pairs (FP64 mma.sync two-qubit blocks)" if args.engine == "pairs"
                            else "k_staged<double,12>") + f" (one read+write of the {16 << nq >> 30} GiB state per launch)",
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "per_launch_bytes": per_launch_bytes, "launches_per_step": passes,

@@ -47,9 +47,10 @@ typedef enum svb_engine {
                                  staged for n >= 10 (FP32: 11), per-gate below */
     SVB_ENGINE_PER_GATE = 1,  /* one HBM sweep per elementary gate, as the reference */
     SVB_ENGINE_STAGED = 2,    /* many gates per HBM sweep through a shared-memory tile */
-    SVB_ENGINE_FUSED = 3,     /* gates fused into dense k-qubit blocks (FP32 only) */
-    SVB_ENGINE_PAIRS = 4      /* FP64 two-qubit blocks on the FP64 tensor cores (FP64, n >= 12,
-                                 no SRN) */
+    SVB_ENGINE_FUSED = 3,     /* gates fused into dense k-qubit blocks (FP32 only); circuits of
+                                 mostly phases run as butterflies when no width is asked for */
+    SVB_ENGINE_PAIRS = 4      /* FP64 two-qubit blocks on the FP64 tensor cores, or butterflies
+                                 in registers where those are faster (FP64, n >= 12, no SRN) */
 } svb_engine;
 
 /* One gate: the fields of the reference's class Gate (svsim_nvgpu_sin.cuh:99-188)
@@ -89,9 +90,10 @@ typedef struct svb_plan_info {
     double   moved_bytes;      /* bytes the plan reads+writes in HBM per run */
     uint64_t plan_bytes;       /* bytes of plan descriptors uploaded by svb_set_circuit */
     int      engine;           /* engine the plan was built for */
-    int      tile_bits;        /* local qubits per tile (staged engine) */
+    int      tile_bits;        /* local qubits per tile */
     uint64_t n_blocks;         /* tensor-core blocks per run: two-qubit blocks of the pair
-                                  engine, fused blocks of the fused engine; 0 otherwise */
+                                  engine, fused blocks of the fused engine; 0 otherwise, and
+                                  where either runs its butterfly form */
 } svb_plan_info;
 
 typedef struct svb_sim svb_sim;

@@ -13,6 +13,7 @@
 #include <mutex>
 #include <string>
 
+#include "bfly.h"
 #include "svb_internal.h"
 
 namespace svb {
@@ -81,6 +82,8 @@ void free_plan(Sim* s)
     cudaFree(s->dpairs.gates);
     s->dpairs = DevPairBuffers{};
     s->pairs = PairPlan{};
+    s->bfly = false;
+    s->dbfly = DevBfBuffers{};
     s->fused = FusedPlan{};
     s->eops.clear();
     s->gates.clear();
@@ -91,6 +94,7 @@ void free_plan(Sim* s)
 void free_scratch(Sim* s)
 {
     free_adjoint_scratch(s->adj);
+    release(s->plan_buf);
     cudaFree(s->mscr.cdf);
     cudaFree(s->mscr.uniforms);
     cudaFree(s->mscr.samples);
@@ -148,6 +152,16 @@ bool staged_supported(int precision, int M)
 svb_status launch_all(Sim* s, cudaStream_t st)
 {
     const int n = (int)s->n;
+    if (s->bfly) {
+        for (size_t p = 0; p < s->info.n_passes; p++) {
+            cudaError_t e = dispatch_prec(s->precision, [&](auto t) {
+                using T = decltype(t);
+                return launch_bfly_pass<T>(s->state, n, (int)p, s->dbfly, st);
+            });
+            if (e != cudaSuccess) return cuda_fail(e, "butterfly pass launch");
+        }
+        return SVB_OK;
+    }
     if (s->engine == SVB_ENGINE_FUSED) {
         const FusedPlan& F = s->fused;
         if (F.k == F6_K) {
@@ -523,7 +537,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         if (it != g_tuned.end()) {
             engine = it->second.engine;
             if (it->second.tile_bits) M = it->second.tile_bits;
-            if (it->second.fusion_width) fusion = it->second.fusion_width;
+            if (engine == SVB_ENGINE_FUSED) fusion = it->second.fusion_width;
         }
     }
     if (has_m4) {
@@ -576,7 +590,24 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     s->info.state_bytes = sb;
     s->info.model_bytes = 2.0 * sb * sweeps;
     s->info.engine = engine;
-    if (engine == SVB_ENGINE_FUSED) {
+    // the butterfly form of the pair engine (FP64) and, where no fusion width is asked for, of
+    // the fused engine (FP32), for the circuits it is faster on
+    if ((engine == SVB_ENGINE_PAIRS || (engine == SVB_ENGINE_FUSED && fusion == 0)) &&
+        bfly_preferred(s->eops, n, s->precision)) {
+        BfPlan B;
+        plan_bfly(s->eops, n, s->precision, B, true);
+        // an earlier circuit's kernels may still read the buffer, on any stream
+        SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+        SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly), "plan upload");
+        s->bfly = true;
+        s->info.n_passes = B.passes.size();
+        s->info.tile_bits = B.tile_bits;
+        s->info.n_blocks = 0;
+        s->info.plan_bytes = B.passes.size() * sizeof(BfPass) + B.ops.size() * sizeof(BfOp) +
+                             B.rels.size() * sizeof(BfRelayout) +
+                             B.coefs.size() * (s->precision == SVB_FP64 ? sizeof(double) : sizeof(float));
+        s->info.moved_bytes = 2.0 * sb * (double)B.passes.size();
+    } else if (engine == SVB_ENGINE_FUSED) {
         const int k = fusion ? fusion : FT_DEFAULT_K;
         if (k == F6_K) plan_fused6(s->eops, n, s->fused);
         else plan_fused(s->eops, n, k, s->fused);
@@ -939,8 +970,10 @@ extern "C" svb_status svb_autotune(svb_sim* s, const svb_gate* gates, size_t n_g
         if (n >= M) cands.push_back({SVB_ENGINE_STAGED, M, 0});
     if (n >= PR_TILE_BITS && matrices) {
         if (fp64) cands.push_back({SVB_ENGINE_PAIRS, 0, 0});
-        else
+        else {
+            if (bfly_preferred(eops, n, s->precision)) cands.push_back({SVB_ENGINE_FUSED, 0, 0});
             for (int k = FT_MIN_K; k <= FT_MAX_K; k++) cands.push_back({SVB_ENGINE_FUSED, 0, k});
+        }
     }
     // the prefix timed: the whole circuit up to 360 gates (the choice holds for the structure)
     const size_t P = std::min<size_t>(n_gates, 360);

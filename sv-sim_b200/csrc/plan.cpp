@@ -39,7 +39,10 @@ OpInfo info_of(const EOp& e, uint64_t all)
 {
     OpInfo r;
     r.need2 = -1;
-    if (e.form == F_M4) {
+    if (e.form == F_PP) {
+        r.touch = bit(e.q) | bit(e.c);
+        r.need = -1;
+    } else if (e.form == F_M4 || e.form == F_SWAP) {
         r.touch = bit(e.q) | bit(e.c);
         r.need = (int)e.q;
         r.need2 = (int)e.c;

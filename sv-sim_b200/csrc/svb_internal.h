@@ -42,6 +42,9 @@ enum Form : uint8_t {
     F_CX,       // CX_GATE :779      swap (c=1,t=0) <-> (c=1,t=1)
     F_M4,       // general 4x4 complex matrix on (q: bit 0, c: bit 1), entries in a side
                 // table (EOp::mat); density-matrix superoperators; pair and per-gate only
+    // made by the butterfly planner from sequences of the others
+    F_PP,       // phase m[0..1] where the values of q and c are equal, m[2..3] where not
+    F_SWAP,     // exchange of qubits q and c
     F_COUNT
 };
 
@@ -345,6 +348,18 @@ bool fusable(const std::vector<EOp>& ops);
 void plan_fused(const std::vector<EOp>& ops, int n, int k, FusedPlan& plan);
 void plan_fused6(const std::vector<EOp>& ops, int n, FusedPlan& plan);
 
+struct BfPlan;                           // butterfly engine (bfly.h)
+struct BfPass;
+struct BfOp;
+struct BfRelayout;
+struct DevBfBuffers {
+    BfPass* passes = nullptr;
+    BfOp* ops = nullptr;
+    BfRelayout* rels = nullptr;
+    void* coefs = nullptr;               // double or float, as the state
+    size_t smem_bytes = 0;
+};
+
 struct DevFusedBuffers {
     FusedPass* passes = nullptr;
     FusedBlock* blocks = nullptr;
@@ -504,6 +519,9 @@ struct Sim {
     DevFusedBuffers dfused;
     PairPlan pairs;
     DevPairBuffers dpairs;
+    bool bfly = false;             // the pair or fused engine's plan is a butterfly plan
+    DevBfBuffers dbfly;            // into bfly_buf
+    GrowBuf plan_buf;              // the butterfly plan, kept from circuit to circuit
     bool have_circuit = false;
     cudaGraphExec_t graph = nullptr;
     cudaStream_t capture_stream = nullptr;

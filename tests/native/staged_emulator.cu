@@ -647,3 +647,154 @@ extern "C" int emu_fused_conflicts(uint32_t n, const svb_gate* gates, size_t n_g
     for (int i = 0; i < 4; i++) out[i] = ins[i] > 0 ? wf[i] / ins[i] : 0.0;
     return 0;
 }
+
+// ---- butterfly plans -----------------------------------------------------------------
+// Executes a butterfly plan (plan_bfly) thread by thread with the kernel's own op
+// application and slot arithmetic (bfly_core.cuh), starting from the given state, in the
+// state's precision.  Checks that loads, redistributions and stores are bijections.
+#include "bfly_core.cuh"
+
+namespace {
+
+template <typename T>
+int run_bfly(int n, const BfPlan& plan, std::vector<typename VecOf<T>::type>& sv)
+{
+    using U = BfUnit<T>;
+    constexpr bool packed = BfScalar<T>::packed;
+    constexpr int UNITS = 1 << BF_UNIT_BITS;
+    std::vector<U> regs((size_t)UNITS), sm(UNITS);
+    std::vector<BfPhase> ph(BF_THREADS);
+    std::vector<int> seen(UNITS);
+    std::vector<T> coefs(plan.coefs.begin(), plan.coefs.end());
+    if constexpr (packed) coefs = bfly_coefs32(plan);
+    const uint64_t tiles = 1ull << (n - plan.tile_bits);
+    for (const BfPass& P : plan.passes) {
+        if (bfly_smem(P.n_ops, P.n_rel, P.n_coef, packed) > BF_SMEM_CAP) return -3;
+        std::vector<int> all_in(sv.size(), 0), all_out(sv.size(), 0);
+        for (uint64_t tile = 0; tile < tiles; tile++) {
+            uint64_t base = 0;
+            for (int j = 0; j < P.n_nonlocal; j++) base |= ((tile >> j) & 1ull) << P.nonlocal_q[j];
+            for (int t = 0; t < BF_THREADS; t++) {
+                ph[t].own = make_double2(1.0, 0.0);
+                for (int k = 0; k < BF_NR; k++) {
+                    const uint64_t g = base | (bf_thr(P.in_thr, t) ^ bf_comb(P.in_reg, k));
+                    if (g >= sv.size() || all_in[g]++) return -2;
+                    U& u = regs[(size_t)t * BF_NR + k];
+                    if constexpr (packed) {
+                        if (g & 1) return -2;
+                        u.re = f2_make(sv[g].x, sv[g + 1].x);
+                        u.im = f2_make(sv[g].y, sv[g + 1].y);
+                    } else {
+                        u.re = sv[g].x;
+                        u.im = sv[g].y;
+                    }
+                }
+            }
+            uint64_t flips = 0;
+            for (int i = 0; i < P.n_tile_masks; i++) flips |= (uint64_t)bf_parity64(P.tile_mask[i] & base) << i;
+            for (int o = 0; o < P.n_ops; o++) {
+                const BfOp& op = plan.ops[P.op_begin + o];
+                if ((op.kind == BF_END) != (o + 1 == P.n_ops)) return -7;
+                if (op.kind == BF_END) break;
+                if (op.kind == BF_ROT) {
+                    for (int t = 0; t < BF_THREADS; t++) bf_apply_rot<T>(op, &regs[(size_t)t * BF_NR], t, flips);
+                    continue;
+                }
+                if (op.kind != BF_RELAYOUT) {
+                    for (int t = 0; t < BF_THREADS; t++)
+                        bf_apply<T>(op, coefs.data() + P.coef_begin, &regs[(size_t)t * BF_NR], &ph[t], t, flips);
+                    continue;
+                }
+                const BfRelayout& R = plan.rels[P.rel_begin + op.lay];
+                std::fill(seen.begin(), seen.end(), 0);
+                for (int t = 0; t < BF_THREADS; t++) {
+                    for (int k = 0; k < BF_NR; k++) {
+                        const uint32_t w = bf_thr(R.wthr, t) ^ bf_comb(R.wreg, k);
+                        if (w >= UNITS || seen[w]++) return -2;
+                        sm[w] = regs[(size_t)t * BF_NR + k];
+                    }
+                }
+                std::fill(seen.begin(), seen.end(), 0);
+                for (int t = 0; t < BF_THREADS; t++)
+                    for (int k = 0; k < BF_NR; k++) {
+                        const uint32_t r = bf_thr(R.rthr, t) ^ bf_comb(R.rreg, k);
+                        if (r >= UNITS || seen[r]++) return -2;
+                        regs[(size_t)t * BF_NR + k] = sm[r];
+                    }
+            }
+            const auto scale = BfScalar<T>::dup(coefs[P.coef_begin + P.n_coef - 1]);
+            uint64_t flip = 0;
+            for (int f = 0; f < P.n_flips; f++)
+                if (bf_parity64(P.flips[f].tile & base)) flip ^= P.flips[f].off;
+            for (int t = 0; t < BF_THREADS; t++) {
+                if (ph[t].own.x != 1.0 || ph[t].own.y != 0.0) return -6;   // not flushed
+                for (int k = 0; k < BF_NR; k++) {
+                    const uint64_t g = base | (flip ^ bf_thr(P.out_thr, t) ^ bf_comb(P.out_reg, k));
+                    if (g >= sv.size() || all_out[g]++) return -2;
+                    U u = regs[(size_t)t * BF_NR + k];
+                    u.re = BfScalar<T>::mul(u.re, scale);
+                    u.im = BfScalar<T>::mul(u.im, scale);
+                    if constexpr (packed) {
+                        if (g & 1) return -2;
+                        f2_split(u.re, sv[g].x, sv[g + 1].x);
+                        f2_split(u.im, sv[g].y, sv[g + 1].y);
+                    } else {
+                        sv[g].x = u.re;
+                        sv[g].y = u.im;
+                    }
+                }
+            }
+            // whole 64-byte runs: the units of lanes 0..3 of every slot are neighbours
+            for (int t = 0; t < BF_THREADS; t += 4)
+                for (int l = 1; l < 4; l++) {
+                    const uint64_t run = packed ? 7 : 3;
+                    if (((bf_thr(P.in_thr, t) ^ bf_thr(P.in_thr, t + l)) & ~run) ||
+                        ((bf_thr(P.out_thr, t) ^ bf_thr(P.out_thr, t + l)) & ~run)) return -4;
+                }
+        }
+    }
+    return 0;
+}
+
+}  // namespace
+
+// (re, im) <- circuit applied to (re, im).  stats: passes, gates, diagonal ops, register
+// moves, relayouts, eight-lane shared-memory phases with bank conflicts, all phases.
+extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, int precision, int tune, int execute,
+                            double* re, double* im, uint64_t* stats)
+{
+    std::vector<EOp> eops;
+    for (size_t i = 0; i < n_gates; i++)
+        if (!lower_gate(gates[i], (int32_t)i, eops)) return -1;
+    if (!bfly_supported(eops, (int)n, precision)) return -5;
+    BfPlan plan;
+    plan_bfly(eops, (int)n, precision, plan, tune != 0);
+    stats[0] = plan.passes.size();
+    stats[1] = plan.n_gates2;
+    stats[2] = plan.n_diags;
+    stats[3] = plan.n_moves;
+    stats[4] = plan.rels.size();
+    stats[5] = stats[6] = 0;
+    for (const BfRelayout& R : plan.rels)
+        for (int side = 0; side < 2; side++) {
+            const uint16_t* thr = side ? R.rthr : R.wthr;
+            uint32_t groups = 0;
+            for (int l = 0; l < 8; l++) groups |= 1u << (bf_thr(thr, l) & 7);
+            stats[5] += groups != 0xff;
+            stats[6]++;
+        }
+    if (!execute) return 0;
+    const uint64_t dim = 1ull << n;
+    if (precision == SVB_FP64) {
+        std::vector<double2> sv(dim);
+        for (uint64_t i = 0; i < dim; i++) sv[i] = make_double2(re[i], im[i]);
+        const int rc = run_bfly<double>((int)n, plan, sv);
+        for (uint64_t i = 0; i < dim; i++) { re[i] = sv[i].x; im[i] = sv[i].y; }
+        return rc;
+    }
+    std::vector<float2> sv(dim);
+    for (uint64_t i = 0; i < dim; i++) sv[i] = make_float2((float)re[i], (float)im[i]);
+    const int rc = run_bfly<float>((int)n, plan, sv);
+    for (uint64_t i = 0; i < dim; i++) { re[i] = sv[i].x; im[i] = sv[i].y; }
+    return rc;
+}

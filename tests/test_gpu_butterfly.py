@@ -1,0 +1,98 @@
+"""The butterfly form of the pair (FP64) and fused (FP32) engines on the GPU, against the
+per-gate engine, which is the reference CPU's arithmetic bit for bit."""
+import numpy as np
+import pytest
+
+from svsim_b200 import circuits, gates as G
+from test_plan import phase_circuit
+
+pytestmark = pytest.mark.gpu
+
+
+def qft(n, seed):
+    rng = np.random.default_rng(seed)
+    gl = [G.U3(*rng.uniform(0, 6, 3), q) for q in range(n)]
+    for i in range(n - 1, -1, -1):
+        gl.append(G.H(i))
+        gl += [G.CU1(np.pi / (1 << (i - j)), j, i) for j in range(i - 1, -1, -1)]
+    return G.to_array(gl + [G.SWAP(q, n - 1 - q) for q in range(n // 2)])
+
+
+def swaps(n):
+    """Only label changes: passes without a redistribution, whose stores permute the tile."""
+    return G.to_array([G.SWAP(q, n - 1 - q) for q in range(n // 2)] + [G.CZ(0, n - 1)])
+
+
+@pytest.mark.parametrize("n,precision,make", [
+    (12, 0, phase_circuit), (13, 1, qft), (17, 0, phase_circuit), (20, 0, qft), (20, 1, qft), (23, 0, qft), (24, 1, qft),
+    (14, 0, lambda n, s: swaps(n)), (24, 0, lambda n, s: swaps(n)), (23, 1, lambda n, s: swaps(n)),
+    (25, 0, lambda n, s: circuits.random_matching_circuit(n, 3, seed=s))])
+def test_matches_the_per_gate_engine(n, precision, make):
+    """From a random state, one tile to many tiles per CTA, run twice (the second time as a
+    replayed graph), the second on a stream of its own: 2-norm error within one rounding a
+    gate in quadrature, times 8."""
+    import torch
+    from svsim_b200 import _native as nat
+    g = make(n, n)
+    h = nat.Handle(n, 0, precision)
+    ref = nat.Handle(n, 0, nat.SVB_FP64)
+    ref.set_engine(nat.ENGINE_PER_GATE)
+    h.set_circuit(g)
+    info = h.plan_info()
+    assert info.engine == (nat.ENGINE_FUSED if precision else nat.ENGINE_PAIRS) and info.n_blocks == 0
+    ref.set_circuit(g)
+    if n <= 20:
+        rng = np.random.default_rng(n)
+        st = rng.standard_normal((2, 1 << n))
+        st /= np.sqrt((st ** 2).sum())
+        h.set_state(st[0], st[1])
+        ref.set_state(st[0], st[1])
+    stream = torch.cuda.Stream()
+    for s in (0, stream.cuda_stream):
+        h.run(s)
+        h.sync()
+        ref.run()
+        ref.sync()
+    eps = 1.2e-7 if precision else 2.2e-16
+    bound = 8 * eps * np.sqrt(2 * max(len(g), 100))
+    a = torch.as_tensor(Dev(h), device="cuda").double()
+    b = torch.as_tensor(Dev(ref), device="cuda")
+    assert float(torch.linalg.vector_norm(a - b)) <= bound * float(torch.linalg.vector_norm(b))
+
+
+class Dev:
+    """A handle's amplitudes as torch sees them, no copy."""
+
+    def __init__(self, h):
+        ptr, prec = h.device_ptr()
+        self.h = h
+        self.__cuda_array_interface__ = {"shape": (2 << h.n,), "typestr": "<f8" if prec == 0 else "<f4", "version": 3,
+                                         "data": (ptr, False)}
+
+
+def test_routes(oracle):
+    """Which circuits go where: phase-rich ones to butterflies, random U3 + CX below 25 qubits
+    and FP32 circuits with a fusion width to the tensor cores, SRN to the staged engine."""
+    from svsim_b200 import _native as nat
+    h = nat.Handle(16, 0, nat.SVB_FP64)
+    h.set_circuit(circuits.random_matching_circuit(16, 4, seed=1))
+    assert h.plan_info().n_blocks > 0
+    h.set_circuit(qft(16, 1))
+    assert h.plan_info().n_blocks == 0 and h.plan_info().engine == nat.ENGINE_PAIRS
+    f = nat.Handle(16, 0, nat.SVB_FP32)
+    f.set_circuit(qft(16, 1))
+    assert f.plan_info().n_blocks == 0 and f.plan_info().engine == nat.ENGINE_FUSED
+    f.set_engine(nat.ENGINE_FUSED, 0, 4)
+    f.set_circuit(qft(16, 1))
+    assert f.plan_info().n_blocks > 0
+    h.set_circuit(G.to_array(G.from_array(qft(16, 1)) + [G.SRN(0)]))
+    assert h.plan_info().engine == nat.ENGINE_STAGED
+    # a new circuit while the last one may still run reuses the plan buffer
+    h.set_circuit(qft(16, 2))
+    h.reset()
+    h.run()
+    h.set_circuit(qft(16, 3))
+    h.run()
+    re, im = h.get_state()
+    want = oracle.run(16, np.concatenate([qft(16, 2), qft(16, 3)]))
+    assert np.max(np.abs(re - want[0])) < 1e-13 and np.max(np.abs(im - want[1])) < 1e-13

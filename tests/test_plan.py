@@ -392,3 +392,88 @@ def test_pair_plan_keeps_the_cheaper_pass_cut(emu, n, depth, seed):
     assert plan_cost(both) <= plan_cost(one) + 1e-9
     if n == 30:
         assert int(one[0]) == 50 and int(both[0]) == 48 and plan_cost(both) < plan_cost(one)
+
+
+def phase_circuit(n, seed, reps=2):
+    """Controlled phases, CZ, RZZ and SWAPs between layers of every kind of one-qubit gate:
+    the sequences the butterfly planner shortens, whole and interrupted."""
+    rng = np.random.default_rng(seed)
+    gl = G.from_array(circuits.random_matching_circuit(n, 1, seed=seed))
+    for _ in range(reps):
+        for a in range(n):
+            gl.append(G.H(a))
+            for b in rng.choice(n, size=min(4, n), replace=False):
+                if int(b) == a:
+                    continue
+                t = float(rng.uniform(-3, 3))
+                gl.append([lambda: G.CU1(t, a, int(b)), lambda: G.CZ(a, int(b)), lambda: G.RZZ(t, a, int(b)),
+                           lambda: G.SWAP(a, int(b)), lambda: G.CX(a, int(b)), lambda: G.CRZ(t, a, int(b)),
+                           lambda: G.RXX(t, a, int(b))][int(rng.integers(7))]())
+            gl.append([G.X, G.T, G.Y, G.SDG][a % 4](int(rng.integers(n))))
+    return G.to_array(gl)
+
+
+def run_bfly(lib, n, gates, precision, tune=1, seed=3):
+    rng = np.random.default_rng(seed)
+    st = rng.standard_normal((2, 1 << n))
+    st /= np.sqrt((st ** 2).sum())
+    re, im = st[0].copy(), st[1].copy()
+    stats = (ctypes.c_uint64 * 8)()
+    rc = lib.emu_bfly_run(n, gates.ctypes.data, ctypes.c_size_t(len(gates)), precision, tune, 1, re.ctypes.data_as(_dp),
+                          im.ctypes.data_as(_dp), stats)
+    return rc, (re, im), st, list(stats)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("n,kind", [(12, "matching"), (13, "matching"), (16, "matching"), (13, "phases"), (15, "phases"),
+                                    (13, "every"), (14, "every"), (14, "ansatz"), (15, "long")])
+def test_butterfly_plan_from_random_states(emu, oracle, n, kind, precision):
+    """The butterfly engine's plans, run thread by thread with the kernel's own arithmetic,
+    from a random state: every op it takes (all but SRN and R), one tile and many, passes with
+    and without redistributions, and circuits long enough to be cut at a pass's limits.  FP64
+    within 8 ulps of a unit-norm state per hundred gates, FP32 within its own rounding."""
+    if precision == 1 and n < 13:
+        pytest.skip("an FP32 tile has 13 qubits")
+    if kind == "matching":
+        g = circuits.random_matching_circuit(n, 8, seed=n)
+    elif kind == "phases":
+        g = phase_circuit(n, seed=n)
+    elif kind == "ansatz":
+        g = circuits.hardware_efficient_ansatz(n, 4).gates
+    elif kind == "long":
+        g = np.concatenate([phase_circuit(n, seed=s, reps=6) for s in range(3)])
+    else:
+        g = mixed_circuit(n, 2, seed=n)
+        g = g[(g["op"] != G.OP["SRN"]) & (g["op"] != G.OP["R"])]
+    want = None
+    for tune in (0, 1):
+        rc, got, st, stats = run_bfly(emu, n, g, precision, tune)
+        assert rc == 0 and stats[0] >= 1
+        if want is None:
+            want = oracle.run(n, g, state=(st[0], st[1]))
+        err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+        # 2-norm error: one rounding (eps / 2 of the norm at most) a gate, in quadrature, times 8
+        eps = 2.2e-16 if precision == 0 else 1.2e-7
+        assert err <= 8 * eps * np.sqrt(max(len(g), 100)), (tune, err)
+
+
+def test_butterfly_plan_rejects_what_it_cannot_split(emu):
+    """SRN is not complex-linear, R not unitary: both stay on the other engines, as do states
+    smaller than a tile."""
+    for n, gl, precision in ((13, [G.SRN(1)], 0), (13, [G.R(0.5, 1)], 0), (11, [G.H(0)], 0), (12, [G.H(0)], 1)):
+        assert run_bfly(emu, n, G.to_array(gl), precision)[0] == -5
+
+
+@pytest.mark.parametrize("theta", [0.0, np.pi, 2 * np.pi, np.pi - 1e-9, 1e-9])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_butterfly_plan_at_degenerate_angles(emu, oracle, theta, precision):
+    """Gates whose split has a zero or vanishing diagonal (p = cos(theta / 2)): the scaled form."""
+    n = 13
+    gl = []
+    for q in range(n):
+        gl += [G.U3(theta, 0.3 * q, 1.1, q), G.CX(q, (q + 1) % n), G.RX(theta, (q + 3) % n), G.CX((q + 3) % n, q)]
+    g = G.to_array(gl)
+    rc, got, st, _ = run_bfly(emu, n, g, precision)
+    want = oracle.run(n, g, state=(st[0], st[1]))
+    err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+    assert rc == 0 and err <= 8 * (2.2e-16 if precision == 0 else 1.2e-7) * 10
