@@ -84,6 +84,8 @@ void free_plan(Sim* s)
     s->pairs = PairPlan{};
     s->bfly = false;
     s->dbfly = DevBfBuffers{};
+    s->small_ops = nullptr;
+    s->small_mats = nullptr;
     s->fused = FusedPlan{};
     s->eops.clear();
     s->gates.clear();
@@ -197,6 +199,12 @@ svb_status launch_all(Sim* s, cudaStream_t st)
             });
             if (e != cudaSuccess) return cuda_fail(e, "staged pass launch");
         }
+    } else if (s->small_ops) {
+        cudaError_t e = dispatch_prec(s->precision, [&](auto t) {
+            using T = decltype(t);
+            return launch_small<T>(s->state, n, s->small_ops, (int)s->eops.size(), s->small_mats, st);
+        });
+        if (e != cudaSuccess) return cuda_fail(e, "circuit launch");
     } else {
         for (const EOp& op : s->eops) {
             cudaError_t e = dispatch_prec(s->precision, [&](auto t) {
@@ -709,6 +717,30 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         for (const EOp& e : s->eops)
             moved += (e.form == F_CX || (form_is_diag(e.form) && e.form != F_DIAG)) ? sb : 2.0 * sb;
         s->info.moved_bytes = moved;
+        if (n <= SMALL_QUBITS && !s->eops.empty()) {
+            // one launch: the state goes through shared memory once
+            const size_t ob = s->eops.size() * sizeof(SmallOp), mb = s->mats.size() * sizeof(Mat4);
+            std::vector<unsigned char> host(ob + mb);
+            SmallOp* so = reinterpret_cast<SmallOp*>(host.data());
+            for (size_t i = 0; i < s->eops.size(); i++) {
+                const EOp& e = s->eops[i];
+                std::memcpy(so[i].m, e.m, sizeof(so[i].m));
+                so[i].form = e.form;
+                so[i].q = (uint8_t)e.q;
+                so[i].c = (uint8_t)e.c;
+                so[i].mat = e.mat;
+            }
+            if (mb) std::memcpy(host.data() + ob, s->mats.data(), mb);
+            // an earlier circuit's kernel may still read the buffer, on any stream
+            SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+            SVB_CUDA(grow(s->plan_buf, host.size()), "cudaMalloc(plan)");
+            SVB_CUDA(cudaMemcpy(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice), "plan upload");
+            s->small_ops = static_cast<const SmallOp*>(s->plan_buf.p);
+            s->small_mats = reinterpret_cast<const double*>(static_cast<unsigned char*>(s->plan_buf.p) + ob);
+            s->info.n_passes = 1;
+            s->info.plan_bytes = host.size();
+            s->info.moved_bytes = 2.0 * sb;
+        }
     }
     s->have_circuit = true;
     return SVB_OK;

@@ -88,6 +88,100 @@ k_cx(typename VecOf<T>::type* __restrict__ sv, uint64_t quarter, int c, int t)
     }
 }
 
+// States of up to SMALL_QUBITS qubits: the whole circuit in one launch of one CTA, the state
+// in shared memory, one barrier per op.  The arithmetic is k_eop_pairs' and k_cx's, so the
+// states stay bit-identical.  A launch per op cost 3 us for about 0.1 us of work (a 6-qubit
+// circuit of 60 ops: 180 us of kernels).  Ops are staged 32 at a time.
+constexpr int SMALL_STAGE = 32;
+
+template <typename T>
+__global__ void __launch_bounds__(512)
+k_small(typename VecOf<T>::type* __restrict__ sv, int n, const SmallOp* __restrict__ ops, int n_ops,
+        const double* __restrict__ mats)
+{
+    using V = typename VecOf<T>::type;
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    __shared__ SmallOp so[SMALL_STAGE];
+    V* s = reinterpret_cast<V*>(small_smem);
+    const uint32_t dim = 1u << n, tid = threadIdx.x, nt = blockDim.x;
+    for (uint32_t i = tid; i < dim; i += nt) s[i] = sv[i];
+    for (int o0 = 0; o0 < n_ops; o0 += SMALL_STAGE) {
+        const int cnt = n_ops - o0 < SMALL_STAGE ? n_ops - o0 : SMALL_STAGE;
+        const uint4* src = reinterpret_cast<const uint4*>(ops + o0);
+        for (uint32_t w = tid; w < cnt * (uint32_t)(sizeof(SmallOp) / 16); w += nt) reinterpret_cast<uint4*>(so)[w] = src[w];
+        __syncthreads();
+        for (int o = 0; o < cnt; o++) {
+            const int form = so[o].form, q = so[o].q, c = so[o].c;
+            const uint32_t qd = 1u << q, cd = 1u << c;
+            if (form == F_CX) {
+                const int lo = c < q ? c : q, hi = c < q ? q : c;
+                for (uint32_t i = tid; i < dim / 4; i += nt) {
+                    const uint32_t b = (uint32_t)insert_zero(insert_zero(i, lo), hi) | cd;
+                    const V a0 = s[b], a1 = s[b | qd];
+                    s[b] = a1;
+                    s[b | qd] = a0;
+                }
+            } else if (form == F_M4) {
+                const int lo = c < q ? c : q, hi = c < q ? q : c;
+                const double* m = mats + 32 * (size_t)so[o].mat;
+                for (uint32_t i = tid; i < dim / 4; i += nt) {
+                    const uint32_t b = (uint32_t)insert_zero(insert_zero(i, lo), hi);
+                    const uint32_t at[4] = {b, b | qd, b | cd, b | qd | cd};
+                    V x[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) x[k] = s[at[k]];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        V y;
+                        y.x = y.y = 0;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const T mr = (T)m[r * 8 + 2 * k], mi = (T)m[r * 8 + 2 * k + 1];
+                            y.x += mr * x[k].x - mi * x[k].y;
+                            y.y += mr * x[k].y + mi * x[k].x;
+                        }
+                        s[at[r]] = y;
+                    }
+                }
+            } else {
+                const Coef<T> cf = load_coef<T>(so[o].m);
+                const bool diag = form_is_diag(form), both = !diag || form == F_DIAG;
+                for (uint32_t i = tid; i < dim / 2; i += nt) {
+                    const uint32_t p0 = (uint32_t)insert_zero(i, q);
+                    V a0 = s[p0], a1 = s[p0 | qd];
+                    if (diag) {
+                        diag_one<T>(form, cf, a1);
+                        if (form == F_DIAG) diag_zero<T>(form, cf, a0);
+                    } else {
+                        dense_pair<T>(form, cf, a0, a1);
+                    }
+                    s[p0 | qd] = a1;
+                    if (both) s[p0] = a0;
+                }
+            }
+            __syncthreads();                 // the op's writes, and the stage's last readers
+        }
+    }
+    for (uint32_t i = tid; i < dim; i += nt) sv[i] = s[i];
+}
+
+template <typename T>
+cudaError_t launch_small(void* state, int n, const SmallOp* ops, int n_ops, const double* mats, cudaStream_t s)
+{
+    using V = typename VecOf<T>::type;
+    if (n > SMALL_QUBITS) return cudaErrorInvalidValue;
+    const size_t smem = sizeof(V) << n;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const unsigned threads = n < 6 ? 32u : (n > 10 ? 512u : 1u << (n - 1));
+    k_small<T><<<1, threads, smem, s>>>(static_cast<V*>(state), n, ops, n_ops, mats);
+    return cudaGetLastError();
+}
+template cudaError_t launch_small<double>(void*, int, const SmallOp*, int, const double*, cudaStream_t);
+template cudaError_t launch_small<float>(void*, int, const SmallOp*, int, const double*, cudaStream_t);
+
 static unsigned grid_for(uint64_t items, int threads)
 {
     // enough CTAs to fill 148 SMs several times over, grid-stride beyond that

@@ -392,6 +392,17 @@ struct DevPlanBuffers {
 // one elementary op, one sweep (per-gate engine)
 template <typename T>
 cudaError_t launch_eop(void* state, int n, const EOp& op, cudaStream_t s);
+// the per-gate engine on a state of at most SMALL_QUBITS qubits: all ops in one launch
+constexpr int SMALL_QUBITS = 12;         // 64 KiB of FP64 state in shared memory
+struct alignas(16) SmallOp {             // 80 bytes
+    double m[8];
+    uint8_t form, q, c, pad;
+    int32_t mat;                         // F_M4: its 4x4 matrix
+    uint64_t pad2;
+};
+static_assert(sizeof(SmallOp) == 80, "SmallOp layout");
+template <typename T>
+cudaError_t launch_small(void* state, int n, const SmallOp* ops, int n_ops, const double* mats, cudaStream_t s);
 // one staged pass
 template <typename T>
 cudaError_t launch_staged_pass(void* state, int n, int M, int pass_index,
@@ -521,7 +532,10 @@ struct Sim {
     DevPairBuffers dpairs;
     bool bfly = false;             // the pair or fused engine's plan is a butterfly plan
     DevBfBuffers dbfly;            // into bfly_buf
-    GrowBuf plan_buf;              // the butterfly plan, kept from circuit to circuit
+    GrowBuf plan_buf;              // the butterfly plan's or the small state's ops, kept from
+                                   // circuit to circuit
+    const SmallOp* small_ops = nullptr;   // per-gate engine on a small state: into plan_buf
+    const double* small_mats = nullptr;
     bool have_circuit = false;
     cudaGraphExec_t graph = nullptr;
     cudaStream_t capture_stream = nullptr;
