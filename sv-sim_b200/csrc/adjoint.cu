@@ -20,7 +20,7 @@
 #include <algorithm>
 #include <string>
 
-#include "gate_math.cuh"
+#include "pauli.cuh"
 
 namespace svb {
 
@@ -475,25 +475,8 @@ k_pauli_apply(const double2* __restrict__ psi, double2* __restrict__ out, uint64
     for (int t = threadIdx.x; t < n_terms; t += blockDim.x) sterms[t] = terms[t];
     __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += stride) {
-        double accr = 0.0, acci = 0.0;
-        for (int t = 0; t < n_terms; t++) {
-            const uint64_t j = i ^ sterms[t].x_mask;
-            const double2 b = psi[j];
-            double br = b.x, bi = b.y;
-            if (__popcll(j & sterms[t].z_mask) & 1) { br = -br; bi = -bi; }
-            double tr, ti;
-            switch (__popcll(sterms[t].x_mask & sterms[t].z_mask) & 3) {
-            case 0: tr = br; ti = bi; break;
-            case 1: tr = -bi; ti = br; break;
-            case 2: tr = -br; ti = -bi; break;
-            default: tr = bi; ti = -br; break;
-            }
-            accr += sterms[t].coef * tr;
-            acci += sterms[t].coef * ti;
-        }
-        out[i] = make_double2(accr, acci);
-    }
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += PAULI_U * stride)
+        pauli_apply(psi, out, i, stride, dim, sterms, n_terms);
 }
 
 __global__ void __launch_bounds__(256)
@@ -934,9 +917,9 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
     if ((err = cudaMemcpyAsync(A.final_state.p, s->state, sbytes, cudaMemcpyDeviceToDevice)) != cudaSuccess)
         return fail(err, "final state copy");
     // lambda = H psi, energy = Re <psi|lambda>
-    const unsigned g = adj_grid(dim);
     if (n_terms)
-        k_pauli_apply<<<g, 256, n_terms * sizeof(svb_pauli_term)>>>(
+        k_pauli_apply<<<(unsigned)std::min<uint64_t>((dim + 256 * PAULI_U - 1) / (256 * PAULI_U), 148 * 16), 256,
+                        n_terms * sizeof(svb_pauli_term)>>>(
             static_cast<const double2*>(s->state), lam, dim, dterms, (int)n_terms);
     else
         err = cudaMemset(lam, 0, sbytes);

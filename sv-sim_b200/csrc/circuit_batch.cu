@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "pairs_core.cuh"
+#include "pauli.cuh"
 
 namespace svb {
 namespace {
@@ -244,25 +245,10 @@ __global__ void __launch_bounds__(512) k_cbatch(CbArgs A)
         const uint64_t end = start + CB_CHUNK < dim ? start + CB_CHUNK : dim;
         const V* sv = pool + C.state_off;
         double acc = 0.0;
-        for (uint64_t i = start + lane; i < end; i += 32) {
-            const V a = sv[i];
-            const double ar = (double)a.x, ai = (double)a.y;
-            for (uint32_t t = C.term_begin; t < C.term_end; t++) {
-                const svb_pauli_term P = A.terms[t];
-                const uint64_t j = i ^ P.x_mask;
-                const V b = sv[j];
-                double br = (double)b.x, bi = (double)b.y;
-                if (__popcll(j & P.z_mask) & 1) { br = -br; bi = -bi; }
-                double tr, ti;
-                switch (__popcll(P.x_mask & P.z_mask) & 3) {     // i^(number of Y factors)
-                case 0: tr = br; ti = bi; break;
-                case 1: tr = -bi; ti = br; break;
-                case 2: tr = -br; ti = -bi; break;
-                default: tr = bi; ti = -br; break;
-                }
-                acc += P.coef * (ar * tr + ai * ti);
-            }
-        }
+        const int n_terms = (int)(C.term_end - C.term_begin);
+        if (n_terms > 0)
+            for (uint64_t i = start + lane; i < end; i += 32 * PAULI_U)
+                acc += pauli_energy<T>(sv, i, 32, end, A.terms + C.term_begin, n_terms);
         acc = cb_warp_sum(acc);
         if (lane == 0) A.partial[k] = acc;
     }

@@ -39,7 +39,7 @@
 // States of at most WALK_BLOCKS blocks skip passes 1-3 and 5: the chain walks every block.
 // Every step computes the reference's sequential values themselves, so equal inputs
 // give the reference's samples whatever the summation order of pass 1.
-#include "gate_math.cuh"
+#include "pauli.cuh"
 
 namespace svb {
 namespace {
@@ -641,25 +641,8 @@ k_pauli_expect(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim,
     __syncthreads();
     double acc = 0.0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += stride) {
-        const auto a = sv[i];
-        const double ar = (double)a.x, ai = (double)a.y;
-        for (int t = 0; t < n_terms; t++) {
-            const uint64_t xm = sterms[t].x_mask, zm = sterms[t].z_mask;
-            const uint64_t j = i ^ xm;
-            const auto b = sv[j];
-            double br = (double)b.x, bi = (double)b.y;
-            if (__popcll(j & zm) & 1) { br = -br; bi = -bi; }
-            double tr, ti;
-            switch (__popcll(xm & zm) & 3) {     // i^(number of Y factors)
-            case 0: tr = br; ti = bi; break;
-            case 1: tr = -bi; ti = br; break;
-            case 2: tr = -br; ti = -bi; break;
-            default: tr = bi; ti = -br; break;
-            }
-            acc += sterms[t].coef * (ar * tr + ai * ti);
-        }
-    }
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += PAULI_U * stride)
+        acc += pauli_energy<T>(sv, i, stride, dim, sterms, n_terms);
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
