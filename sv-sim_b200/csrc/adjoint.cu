@@ -55,7 +55,8 @@ constexpr int AT_M = 10;                  // 1,024 amplitudes of psi and of lamb
 constexpr int AT_THREADS = 256;
 constexpr int AT_MAX_LSLOTS = 128;   // derivative slots of one pass at most (a pass with more is split)
 
-enum { AT_C1 = 0, AT_DIAG = 1, AT_CX = 2 };
+// AT_REAL: a real 2x2 (RY, H, X), by k_adj_stages only
+enum { AT_C1 = 0, AT_DIAG = 1, AT_CX = 2, AT_REAL = 3 };
 
 struct AdjTileOp {
     uint8_t kind;      // AT_C1 (target local), AT_DIAG, AT_CX (target local)
@@ -240,46 +241,78 @@ static_assert(sizeof(AdjStage) == 32, "AdjStage layout");
 
 enum { AS_LOC_REG = 0, AS_LOC_THREAD = 1, AS_LOC_TILE = 2 };
 
+// Derivatives.  With psi and lambda both after gate U, Re <lambda_U| dU |psi before U> is
+// Re <lambda| K |psi> with K = dU U^dagger, taken before the gate is undone: for RY K is the
+// real matrix [[0, -1/2], [1/2, 0]] (4 multiply-adds a pair), for U1 i |1><1| (2 an
+// amplitude, and no need for the pair: a differentiated RZ stays a diagonal op that may sit
+// on any qubit).  Forming dU psi by a general 2x2 took 24, and undoing a real or diagonal
+// gate by a general 2x2 twice the multiply-adds: the FP64 pipe was the largest part of the
+// sweep (n = 20 ansatz: a gradient 4.89 ms, now 3.42).
 struct AdjStageOp {
-    uint8_t kind;      // AT_C1, AT_DIAG, AT_CX
+    uint8_t kind;      // AT_C1, AT_DIAG, AT_CX, AT_REAL
     uint8_t j;         // C1 / CX: register bit of the target; DIAG: bit of the qubit in its location
     uint8_t c;         // CX: bit of the control in its location
     uint8_t loc;       // DIAG qubit / CX control: AS_LOC_REG, AS_LOC_THREAD or AS_LOC_TILE
-    uint8_t nd;        // derivative slots (AT_C1)
+    uint8_t nd;        // derivative slots (AT_DIAG, AT_REAL: at most one)
     uint8_t pad[3];
     int32_t lslot;
     int32_t pad2;
-    double m[8];
-    double dm[3][8];
+    double m[8];       // inverse: C1 2x2; REAL r00 r01 r10 r11, k; DIAG d0, d1 (2 each)
+    double dm[3][8];   // AT_C1: K of each slot
 };
 static_assert(sizeof(AdjStageOp) % 16 == 0, "AdjStageOp layout");
+// The first 80 bytes of each of a pass's ops are copied into shared memory (up to
+// AS_SMEM_OPS; what is beyond is read from global memory): the op loop waited for a chain of
+// global loads per op.
+constexpr int AS_SMEM_OPS = 96;
+constexpr int AS_HEAD = 5;               // 16-byte words
+
+__device__ __forceinline__ double as_dot(const double2& a, const double2& b) { return a.x * b.x + a.y * b.y; }
 
 template <int J>
-__device__ __forceinline__ void as_c1(double2* vp, double2* vl, const Coef<double>& inv, const double (*dm)[8],
-                                      int nd, double* acc)
+__device__ __forceinline__ double as_deriv_c1(const double2* vp, const double2* vl, const double* k)
+{
+    double acc = 0.0;
+#pragma unroll
+    for (int r = 0; r < AS_R; r++) {
+        if (r & (1 << J)) continue;
+        const double2 s0 = vp[r], s1 = vp[r | (1 << J)];
+        acc += vl[r].x * (k[0] * s0.x - k[1] * s0.y + k[2] * s1.x - k[3] * s1.y);
+        acc += vl[r].y * (k[0] * s0.y + k[1] * s0.x + k[2] * s1.y + k[3] * s1.x);
+        acc += vl[r | (1 << J)].x * (k[4] * s0.x - k[5] * s0.y + k[6] * s1.x - k[7] * s1.y);
+        acc += vl[r | (1 << J)].y * (k[4] * s0.y + k[5] * s0.x + k[6] * s1.y + k[7] * s1.x);
+    }
+    return acc;
+}
+
+template <int J>
+__device__ __forceinline__ void as_c1(double2* v, const Coef<double>& inv)
+{
+#pragma unroll
+    for (int r = 0; r < AS_R; r++)
+        if (!(r & (1 << J))) dense_pair<double>(F_C1, inv, v[r], v[r | (1 << J)]);
+}
+
+// Re <lambda| [[0, -1], [1, 0]] |psi> over the pairs of register bit J
+template <int J>
+__device__ __forceinline__ double as_deriv_real(const double2* vp, const double2* vl)
+{
+    double acc = 0.0;
+#pragma unroll
+    for (int r = 0; r < AS_R; r++)
+        if (!(r & (1 << J))) acc += as_dot(vl[r | (1 << J)], vp[r]) - as_dot(vl[r], vp[r | (1 << J)]);
+    return acc;
+}
+
+template <int J>
+__device__ __forceinline__ void as_real(double2* v, double r00, double r01, double r10, double r11)
 {
 #pragma unroll
     for (int r = 0; r < AS_R; r++) {
         if (r & (1 << J)) continue;
-        const int r1 = r | (1 << J);
-        double2 s0 = vp[r], s1 = vp[r1];
-        double2 l0 = vl[r], l1 = vl[r1];
-        dense_pair<double>(F_C1, inv, s0, s1);
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            if (d >= nd) break;
-            const double* m = dm[d];
-            const double u0r = m[0] * s0.x - m[1] * s0.y + m[2] * s1.x - m[3] * s1.y;
-            const double u0i = m[0] * s0.y + m[1] * s0.x + m[2] * s1.y + m[3] * s1.x;
-            const double u1r = m[4] * s0.x - m[5] * s0.y + m[6] * s1.x - m[7] * s1.y;
-            const double u1i = m[4] * s0.y + m[5] * s0.x + m[6] * s1.y + m[7] * s1.x;
-            acc[d] += l0.x * u0r + l0.y * u0i + l1.x * u1r + l1.y * u1i;
-        }
-        dense_pair<double>(F_C1, inv, l0, l1);
-        vp[r] = s0;
-        vp[r1] = s1;
-        vl[r] = l0;
-        vl[r1] = l1;
+        const double2 a = v[r], b = v[r | (1 << J)];
+        v[r] = make_double2(r00 * a.x + r01 * b.x, r00 * a.y + r01 * b.y);
+        v[r | (1 << J)] = make_double2(r10 * a.x + r11 * b.x, r10 * a.y + r11 * b.y);
     }
 }
 
@@ -313,25 +346,32 @@ __device__ __forceinline__ void as_swap_ctrl(double2* vp, double2* vl)
     }
 }
 
-template <int J>
-__device__ __forceinline__ void as_diag_reg(double2* vp, double2* vl, const Coef<double>& inv)
+// v *= c + i s
+__device__ __forceinline__ void as_phase(double2& v, double c, double s)
 {
-#pragma unroll
-    for (int r = 0; r < AS_R; r++) {
-        if (r & (1 << J)) {
-            diag_one<double>(F_DIAG, inv, vp[r]);
-            diag_one<double>(F_DIAG, inv, vl[r]);
-        } else {
-            diag_zero<double>(F_DIAG, inv, vp[r]);
-            diag_zero<double>(F_DIAG, inv, vl[r]);
-        }
-    }
+    v = make_double2(c * v.x - s * v.y, c * v.y + s * v.x);
 }
 
-__global__ void __launch_bounds__(AS_THREADS, 3)
+// the diagonal inverse on the amplitudes whose register bit J is 1 (J < 0: on all), after
+// the derivative Re <lambda| i |psi> over them
+template <int J>
+__device__ __forceinline__ double as_diag(double2* vp, double2* vl, double c, double s, bool deriv)
+{
+    double acc = 0.0;
+#pragma unroll
+    for (int r = 0; r < AS_R; r++) {
+        if (J >= 0 && !(r & (1 << (J & 3)))) continue;
+        if (deriv) acc += vl[r].y * vp[r].x - vl[r].x * vp[r].y;
+        as_phase(vp[r], c, s);
+        as_phase(vl[r], c, s);
+    }
+    return acc;
+}
+
+__global__ void __launch_bounds__(AS_THREADS, 4)
 k_adj_stages(double2* __restrict__ psi, double2* __restrict__ lam, const AdjTilePass* __restrict__ passes,
              int pass_index, const AdjStage* __restrict__ stages, const AdjStageOp* __restrict__ ops,
-             const int32_t* __restrict__ lslots, uint64_t tiles, double* __restrict__ partial)
+             const int32_t* __restrict__ lslots, int max_lslots, uint64_t tiles, double* __restrict__ partial)
 {
     extern __shared__ __align__(16) double2 as_sm[];
     __shared__ AdjTilePass P;
@@ -347,6 +387,11 @@ k_adj_stages(double2* __restrict__ psi, double2* __restrict__ lam, const AdjTile
     double2* sp = as_sm;
     double2* sl = as_sm + T;
     double* wsum = reinterpret_cast<double*>(as_sm + 2 * T);      // [local slot][warp]
+    uint4* sops = reinterpret_cast<uint4*>(wsum + max_lslots * WARPS);
+    const int op0 = P.stage_begin < P.stage_end ? stages[P.stage_begin].op_begin : 0;
+    const int op1 = P.stage_begin < P.stage_end ? stages[P.stage_end - 1].op_end : 0;
+    for (int w = tid; w < min(op1 - op0, AS_SMEM_OPS) * AS_HEAD; w += AS_THREADS)
+        sops[w] = __ldg(reinterpret_cast<const uint4*>(ops + op0 + w / AS_HEAD) + w % AS_HEAD);
     for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         uint64_t base = 0;
         for (int j = 0; j < P.n_nonlocal; j++) base |= ((tile >> j) & 1ull) << P.nonlocal_q[j];
@@ -370,43 +415,33 @@ k_adj_stages(double2* __restrict__ psi, double2* __restrict__ lam, const AdjTile
                 vl[r] = sl[l];
             }
             for (int o = S.op_begin; o < S.op_end; o++) {
-                const AdjStageOp& op = ops[o];
-                const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(&op));
+                const uint4* head = o - op0 < AS_SMEM_OPS ? sops + (o - op0) * AS_HEAD
+                                                          : reinterpret_cast<const uint4*>(ops + o);
+                const uint4 hdr = head[0];
+                const double* m = reinterpret_cast<const double*>(head + 1);
                 const int kind = hdr.x & 0xFFu, j = (hdr.x >> 8) & 0xFFu, c = (hdr.x >> 16) & 0xFFu;
                 const int loc = hdr.x >> 24, nd = hdr.y & 0xFFu, lslot = (int)hdr.z;
-                Coef<double> inv;
-                {
-                    const double2* m2 = reinterpret_cast<const double2*>(op.m);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const double2 v = __ldg(m2 + q);
-                        inv.m[2 * q] = v.x;
-                        inv.m[2 * q + 1] = v.y;
+                double acc = 0.0;
+                if (kind == AT_REAL) {
+                    const double r00 = m[0], r01 = m[1], r10 = m[2], r11 = m[3];
+                    if (nd) {
+                        if (j == 0) acc = as_deriv_real<0>(vp, vl);
+                        else if (j == 1) acc = as_deriv_real<1>(vp, vl);
+                        else acc = as_deriv_real<2>(vp, vl);
+                        acc *= m[4];
                     }
-                }
-                if (kind == AT_C1) {
-                    double dm[3][8];
-#pragma unroll
-                    for (int d = 0; d < 3; d++) {
-                        const double2* m2 = reinterpret_cast<const double2*>(op.dm[d]);
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const double2 v = d < nd ? __ldg(m2 + q) : make_double2(0.0, 0.0);
-                            dm[d][2 * q] = v.x;
-                            dm[d][2 * q + 1] = v.y;
-                        }
-                    }
-                    double acc[3] = {0.0, 0.0, 0.0};
-                    if (j == 0) as_c1<0>(vp, vl, inv, dm, nd, acc);
-                    else if (j == 1) as_c1<1>(vp, vl, inv, dm, nd, acc);
-                    else as_c1<2>(vp, vl, inv, dm, nd, acc);
-#pragma unroll
-                    for (int d = 0; d < 3; d++) {
-                        if (d >= nd) break;
-                        double v = acc[d];
-#pragma unroll
-                        for (int sh = 16; sh > 0; sh >>= 1) v += __shfl_xor_sync(0xffffffffu, v, sh);
-                        if (lane == 0) wsum[(lslot + d) * WARPS + warp] = v;
+                    if (j == 0) { as_real<0>(vp, r00, r01, r10, r11); as_real<0>(vl, r00, r01, r10, r11); }
+                    else if (j == 1) { as_real<1>(vp, r00, r01, r10, r11); as_real<1>(vl, r00, r01, r10, r11); }
+                    else { as_real<2>(vp, r00, r01, r10, r11); as_real<2>(vl, r00, r01, r10, r11); }
+                } else if (kind == AT_DIAG) {
+                    // d0 is 1 for every gate of the reference's set
+                    const double pc = m[2], ps = m[3];
+                    if (loc == AS_LOC_REG) {
+                        if (j == 0) acc = as_diag<0>(vp, vl, pc, ps, nd);
+                        else if (j == 1) acc = as_diag<1>(vp, vl, pc, ps, nd);
+                        else acc = as_diag<2>(vp, vl, pc, ps, nd);
+                    } else if (loc == AS_LOC_THREAD ? ((tid >> j) & 1) : ((tile >> j) & 1ull)) {
+                        acc = as_diag<-1>(vp, vl, pc, ps, nd);
                     }
                 } else if (kind == AT_CX) {
                     if (loc == AS_LOC_REG) {
@@ -421,24 +456,34 @@ k_adj_stages(double2* __restrict__ psi, double2* __restrict__ lam, const AdjTile
                             else as_swap_all<2>(vp, vl);
                         }
                     }
-                } else {                     // AT_DIAG
-                    if (loc == AS_LOC_REG) {
-                        if (j == 0) as_diag_reg<0>(vp, vl, inv);
-                        else if (j == 1) as_diag_reg<1>(vp, vl, inv);
-                        else as_diag_reg<2>(vp, vl, inv);
-                    } else {
-                        const bool one = loc == AS_LOC_THREAD ? ((tid >> j) & 1) : ((tile >> j) & 1ull);
+                } else {                     // AT_C1
+                    for (int d = 0; d < nd; d++) {
+                        double k[8];
+                        const double2* k2 = reinterpret_cast<const double2*>(ops[o].dm[d]);
 #pragma unroll
-                        for (int r = 0; r < AS_R; r++) {
-                            if (one) {
-                                diag_one<double>(F_DIAG, inv, vp[r]);
-                                diag_one<double>(F_DIAG, inv, vl[r]);
-                            } else {
-                                diag_zero<double>(F_DIAG, inv, vp[r]);
-                                diag_zero<double>(F_DIAG, inv, vl[r]);
-                            }
+                        for (int q = 0; q < 4; q++) {
+                            const double2 v = __ldg(k2 + q);
+                            k[2 * q] = v.x;
+                            k[2 * q + 1] = v.y;
                         }
+                        double v;
+                        if (j == 0) v = as_deriv_c1<0>(vp, vl, k);
+                        else if (j == 1) v = as_deriv_c1<1>(vp, vl, k);
+                        else v = as_deriv_c1<2>(vp, vl, k);
+#pragma unroll
+                        for (int sh = 16; sh > 0; sh >>= 1) v += __shfl_xor_sync(0xffffffffu, v, sh);
+                        if (lane == 0) wsum[(lslot + d) * WARPS + warp] = v;
                     }
+                    const Coef<double> inv = load_coef<double>(m);
+                    if (j == 0) { as_c1<0>(vp, inv); as_c1<0>(vl, inv); }
+                    else if (j == 1) { as_c1<1>(vp, inv); as_c1<1>(vl, inv); }
+                    else { as_c1<2>(vp, inv); as_c1<2>(vl, inv); }
+                    continue;
+                }
+                if (nd) {
+#pragma unroll
+                    for (int sh = 16; sh > 0; sh >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sh);
+                    if (lane == 0) wsum[lslot * WARPS + warp] = acc;
                 }
             }
 #pragma unroll
@@ -574,6 +619,25 @@ bool deriv_matrix(const EOp& e, int i, double* m)
     }
 }
 
+// d <- d . inv (2x2 complex, C1 layout)
+void times_inverse(double* d, const double* inv)
+{
+    double r[8];
+    for (int i = 0; i < 2; i++)
+        for (int j = 0; j < 2; j++) {
+            double re = 0, im = 0;
+            for (int k = 0; k < 2; k++) {
+                const double ar = d[4 * i + 2 * k], ai = d[4 * i + 2 * k + 1];
+                const double br = inv[4 * k + 2 * j], bi = inv[4 * k + 2 * j + 1];
+                re += ar * br - ai * bi;
+                im += ar * bi + ai * br;
+            }
+            r[4 * i + 2 * j] = re;
+            r[4 * i + 2 * j + 1] = im;
+        }
+    std::memcpy(d, r, sizeof(r));
+}
+
 // U^dagger of an elementary op as an F_C1 / F_DIAG / F_CX op.
 bool inverse_op(const EOp& e, EOp& inv)
 {
@@ -665,7 +729,7 @@ void build_stages(std::vector<AdjTilePass>& tpasses, const std::vector<AdjTileOp
             int32_t e = o;
             for (; e < P.op_end; e++) {
                 const AdjTileOp& t = tops[e];
-                if (t.kind != AT_C1 && t.kind != AT_CX) continue;
+                if (t.kind == AT_DIAG) continue;
                 if (std::find(rp.begin(), rp.end(), (int)t.p) != rp.end()) continue;
                 if (rp.size() == 3) break;
                 rp.push_back(t.p);
@@ -695,7 +759,7 @@ void build_stages(std::vector<AdjTilePass>& tpasses, const std::vector<AdjTileOp
                 std::memcpy(so.m, t.m, sizeof(so.m));
                 std::memcpy(so.dm, t.dm, sizeof(so.dm));
                 uint8_t loc = AS_LOC_REG;
-                if (t.kind == AT_C1) {
+                if (t.kind == AT_C1 || t.kind == AT_REAL) {
                     where(t.p, loc, so.j);
                 } else if (t.kind == AT_CX) {
                     where(t.p, loc, so.j);
@@ -929,6 +993,7 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
 
     // reverse sweep, tiled: the inverse ops in reverse order, cut into passes of TM local
     // qubits; a pass never spans a checkpoint, after which psi is reloaded
+    const bool staged_rev = TM == AT_M;               // with register stages
     std::vector<AdjTilePass> tpasses;
     std::vector<AdjTileOp> tops;
     std::vector<int32_t> tslots;                      // per pass: global slot of each local slot
@@ -945,8 +1010,8 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
             for (size_t kk = kk_hi; kk-- > kk_lo;) {
                 EOp inv;
                 inverse_op(eops[kk], inv);
-                if (n_slot[kk] > 0 && inv.form == F_DIAG) {
-                    // a differentiated op needs its pairs local: as a general 2x2
+                if (n_slot[kk] > 0 && inv.form == F_DIAG && !staged_rev) {
+                    // k_adj_tiles needs a differentiated op's pairs local: as a general 2x2
                     const double d0r = inv.m[0], d0i = inv.m[1], d1r = inv.m[2], d1i = inv.m[3];
                     inv.form = F_C1;
                     const double c1[8] = {d0r, d0i, 0, 0, 0, 0, d1r, d1i};
@@ -980,6 +1045,21 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
                     const size_t kk = orig[i];
                     AdjTileOp t;
                     std::memset(&t, 0, sizeof(t));
+                    if (n_slot[kk] > 0) {
+                        if ((int)(tslots.size() - P.lslot_begin) + n_slot[kk] > AT_MAX_LSLOTS) {
+                            // the warps' sums would not fit: the rest of the ops in a second
+                            // pass over the same layout
+                            P.op_end = (int32_t)tops.size();
+                            P.n_lslots = (int32_t)tslots.size() - P.lslot_begin;
+                            max_lslots = std::max(max_lslots, P.n_lslots);
+                            tpasses.push_back(P);
+                            P.op_begin = (int32_t)tops.size();
+                            P.lslot_begin = (int32_t)tslots.size();
+                        }
+                        t.nd = (uint8_t)n_slot[kk];
+                        t.lslot = (int32_t)tslots.size() - P.lslot_begin;
+                        for (int d = 0; d < n_slot[kk]; d++) tslots.push_back(first_slot[kk] + d);
+                    }
                     if (e.form == F_CX) {
                         t.kind = AT_CX;
                         t.p = (uint8_t)pos[e.q];
@@ -991,23 +1071,19 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
                         if (pos[e.q] >= 0) t.p = (uint8_t)pos[e.q];
                         else { t.flags |= 1; t.tile_bit = (uint8_t)tbit[e.q]; }
                     } else {
-                        if ((int)(tslots.size() - P.lslot_begin) + n_slot[kk] > AT_MAX_LSLOTS) {
-                            // the warps' sums would not fit: the rest of the ops in a second
-                            // pass over the same layout
-                            P.op_end = (int32_t)tops.size();
-                            P.n_lslots = (int32_t)tslots.size() - P.lslot_begin;
-                            max_lslots = std::max(max_lslots, P.n_lslots);
-                            tpasses.push_back(P);
-                            P.op_begin = (int32_t)tops.size();
-                            P.lslot_begin = (int32_t)tslots.size();
-                        }
+                        const uint8_t form = eops[kk].form;
                         t.kind = AT_C1;
                         t.p = (uint8_t)pos[e.q];
                         std::memcpy(t.m, e.m, sizeof(t.m));
-                        t.nd = (uint8_t)n_slot[kk];
-                        t.lslot = (int32_t)tslots.size() - P.lslot_begin;
-                        for (int d = 0; d < n_slot[kk]; d++) tslots.push_back(first_slot[kk] + d);
-                        for (int d = 0; d < n_slot[kk]; d++) deriv_matrix(eops[kk], slots[first_slot[kk] + d].i, t.dm[d]);
+                        for (int d = 0; d < n_slot[kk]; d++) {
+                            deriv_matrix(eops[kk], slots[first_slot[kk] + d].i, t.dm[d]);
+                            if (staged_rev) times_inverse(t.dm[d], e.m);
+                        }
+                        if (staged_rev && (form == F_RY || form == F_H || form == F_X)) {
+                            t.kind = AT_REAL;
+                            for (int i2 = 0; i2 < 4; i2++) t.m[i2] = e.m[2 * i2];
+                            t.m[4] = 0.5;                // K of RY
+                        }
                     }
                     tops.push_back(t);
                 }
@@ -1023,7 +1099,6 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
         }
     }
     // register stages of the reverse passes (tiles of AT_M qubits)
-    const bool staged_rev = TM == AT_M;
     std::vector<AdjStage> stages;
     std::vector<AdjStageOp> sops;
     if (staged_rev) build_stages(tpasses, tops, stages, sops);
@@ -1073,7 +1148,8 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
     double2* psi = static_cast<double2*>(s->state);
     if (staged_rev) {
         static int ctas_per_sm = 0, sms = 0;
-        const size_t smem = (2 * sizeof(double2) << AT_M) + AT_MAX_LSLOTS * (AS_THREADS / 32) * sizeof(double);
+        const size_t smem = (2 * sizeof(double2) << AT_M) + AT_MAX_LSLOTS * (AS_THREADS / 32) * sizeof(double) +
+                            AS_SMEM_OPS * AS_HEAD * 16;
         if (ctas_per_sm == 0) {
             if ((err = cudaFuncSetAttribute(k_adj_stages, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
                     cudaSuccess ||
@@ -1084,14 +1160,15 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
             ctas_per_sm = std::max(ctas_per_sm, 1);
         }
         const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctas_per_sm * sms);
-        const size_t dyn = (2 * sizeof(double2) << AT_M) + (size_t)max_lslots * (AS_THREADS / 32) * sizeof(double);
+        const size_t dyn = (2 * sizeof(double2) << AT_M) + (size_t)max_lslots * (AS_THREADS / 32) * sizeof(double) +
+                           AS_SMEM_OPS * AS_HEAD * 16;
         size_t pi = 0;
         for (const Seg& sg : segs) {
             for (; pi < sg.pass_end; pi++)
                 k_adj_stages<<<grid, AS_THREADS, dyn>>>(psi, lam, static_cast<const AdjTilePass*>(A.rev_passes.p),
                                                         (int)pi, static_cast<const AdjStage*>(A.rev_stages.p),
                                                         static_cast<const AdjStageOp*>(A.rev_sops.p),
-                                                        static_cast<const int32_t*>(A.rev_slots.p), tiles, partial);
+                                                        static_cast<const int32_t*>(A.rev_slots.p), max_lslots, tiles, partial);
             if ((err = cudaGetLastError()) != cudaSuccess) return fail(err, "reverse pass");
             if (sg.ck >= 0 &&
                 (err = cudaMemcpyAsync(psi, ckpts[sg.ck], sbytes, cudaMemcpyDeviceToDevice)) != cudaSuccess)

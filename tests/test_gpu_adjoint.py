@@ -213,3 +213,56 @@ def test_sharded_parameter_points_single_rank(small_ansatz):
         assert e[i] == e_ref and np.array_equal(g[i], g_ref)
         assert abs(e_only[i] - e_ref) <= 1e-12
         assert abs(energy_plain(h, pc, p, terms) - e_ref) <= 1e-12
+
+
+@pytest.mark.parametrize("n", [9, 10, 11, 14])
+def test_every_differentiated_kind(n):
+    """U3, U2, U1, RX, RY, RZ and the composites that contain them, differentiated on low, high
+    and (n > 10) non-local qubits, with fixed real, diagonal and complex gates in between:
+    central differences of the plain path (step 1e-6: 1e-7)."""
+    from svsim_b200 import _native as nat
+    rng = np.random.default_rng(n)
+    gl, idx, k = [], [], 0
+    for layer in range(2):
+        for q in range(n):
+            kind = (q + 3 * layer) % 6
+            a = rng.uniform(-3, 3, 3)
+            g = [G.U3(*a, q), G.U2(a[0], a[1], q), G.U1(a[0], q), G.RX(a[0], q), G.RY(a[0], q), G.RZ(a[0], q)][kind]
+            fields = [(0, 1, 2), (1, 2), (2,), (0,), (0,), (1,)][kind]
+            gl.append(g)
+            idx.append([(k + fields.index(f)) if f in fields else -1 for f in range(3)])
+            k += len(fields)
+        for q in range(0, n - 1, 2):
+            t = float(rng.uniform(-3, 3))
+            g = [G.CX(q, q + 1), G.RZZ(t, q, n - 1 - q if n - 1 - q != q else q + 1), G.CRY(t, q, q + 1), G.CU1(t, q + 1, q)][(q // 2) % 4]
+            gl.append(g)
+            f = {"RZZ": 0, "CRY": 2, "CU1": 2}.get(g.name)
+            row = [-1, -1, -1]
+            if f is not None:
+                row[f] = k
+                k += 1
+            idx.append(row)
+        for q in range(n):
+            gl.append([G.H, G.T, G.X, G.S, G.Y, G.Z, G.W][(q + layer) % 7](q))
+            idx.append([-1, -1, -1])
+    gates = G.to_array(gl)
+    binding = np.zeros(len(gates), dtype=G.PARAM_DTYPE)
+    binding["idx"] = np.array(idx)
+    binding["coef"] = 1.0
+    params = np.zeros(k)
+    for g, row in zip(gates, idx):
+        for f, name in enumerate(("theta", "phi", "lam")):
+            if row[f] >= 0:
+                params[row[f]] = g[name]
+    pc = circuits.ParamCircuit(n, gates, binding, params)
+    terms = circuits.zz_x_hamiltonian(n)
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    _, grad = h.adjoint(gates, binding, k, terms)
+    hp = nat.Handle(n, 0, nat.SVB_FP64)
+    for p in range(k):
+        e = []
+        for s in (1e-6, -1e-6):
+            pp = params.copy()
+            pp[p] += s
+            e.append(energy_plain(hp, pc, pp, terms))
+        assert abs((e[0] - e[1]) / 2e-6 - grad[p]) <= 1e-7, (p, grad[p])
