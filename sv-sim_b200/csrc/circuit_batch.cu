@@ -346,6 +346,8 @@ struct CbPairPlan {
     std::vector<uint32_t> phase_off;
     size_t stage_bytes = 0;
     uint32_t circuits = 0;
+    std::vector<PairPlan> each;          // the circuits' own plans, without their gates
+    std::vector<size_t> gate_at;         // where each one's gates begin
 };
 
 struct CbPlan {
@@ -601,8 +603,13 @@ bool cb_build_plan(const svb_circuit_batch* b, const svb_gate* gates, int MB, bo
         }
         plan.pool_amps += 1ull << n;
         plan.circ.push_back(C);
+        const size_t gate_at = plan.pairs.gates.size();
         if (is_pair[c] && cb_append_pairs(plan.pairs, pp[c], c, n, pair_items)) {
-            plan.moved_bytes += 2.0 * amp * (double)(1ull << n) * (double)pp[c].passes.size();
+            plan.pairs.gate_at.push_back(gate_at);
+            pp[c].gates.clear();
+            pp[c].gates.shrink_to_fit();
+            plan.pairs.each.push_back(std::move(pp[c]));
+            plan.moved_bytes += 2.0 * amp * (double)(1ull << n) * (double)plan.pairs.each.back().passes.size();
             continue;
         }
         const int M = std::min(n, MB);
@@ -636,6 +643,38 @@ bool cb_build_plan(const svb_circuit_batch* b, const svb_gate* gates, int MB, bo
         plan.pairs.items.insert(plan.pairs.items.end(), v.begin(), v.end());
         plan.pairs.phase_off.push_back((uint32_t)plan.pairs.items.size());
     }
+    return true;
+}
+
+// New angles for a batch whose circuits all run on the pair engine: every circuit lowered and
+// planned with the cut its plan was made with, on the host threads, its structure compared
+// and its gate fragments copied to the upload buffer.  (Building the whole batch plan again,
+// one circuit's lowering after the other, with both cuts of each circuit, its work items and
+// three copies of the fragments, took 13 ms of the 44 of 64 circuits of 20 qubits.)  False,
+// with nothing changed, if a plan came out different.
+bool cb_replan_pairs(svb_circuit_batch* b, const svb_gate* gates)
+{
+    const CbPairPlan& old = b->plan.pairs;
+    std::vector<PairPlan> fresh(b->n_circ);
+    std::vector<char> ok(b->n_circ, 0);
+    auto same = [](const auto& x, const auto& y) {
+        return x.size() == y.size() && (x.empty() || std::memcmp(x.data(), y.data(), x.size() * sizeof(x[0])) == 0);
+    };
+    cb_parallel_for(b->n_circ, [&](size_t c) {
+        std::vector<EOp> eops;
+        eops.reserve(2 * (b->gate_off[c + 1] - b->gate_off[c]));
+        for (uint64_t g = b->gate_off[c]; g < b->gate_off[c + 1]; g++) lower_gate(gates[g], (int32_t)g, eops);
+        const PairPlan& was = old.each[c];
+        PairPlan& now = fresh[c];
+        const size_t end = c + 1 < b->n_circ ? old.gate_at[c + 1] : old.gates.size();
+        ok[c] = plan_pairs_cut(eops, (int)b->n[c], now, nullptr, was.seeds) && same(now.passes, was.passes) &&
+                same(now.ops, was.ops) && same(now.layouts, was.layouts) && now.gates.size() == end - old.gate_at[c];
+    });
+    if (std::find(ok.begin(), ok.end(), 0) != ok.end()) return false;
+    cb_parallel_for(b->n_circ, [&](size_t c) {
+        if (!fresh[c].gates.empty())
+            std::memcpy(b->h_pgates + old.gate_at[c], fresh[c].gates.data(), fresh[c].gates.size() * sizeof(double));
+    });
     return true;
 }
 
@@ -950,6 +989,14 @@ svb_status svb_cbatch_run(svb_circuit_batch* b, const svb_gate* gates, double* e
         for (uint64_t g = 0; g < b->gate_off[b->n_circ]; g++)
             if (gates[g].op != b->gates[g].op || std::memcmp(gates[g].qb, b->gates[g].qb, sizeof(gates[g].qb)) != 0)
                 return cb_invalid("svb_cbatch_run: gate " + std::to_string(g) + " differs from the batch's structure");
+        if (b->plan.pairs.each.size() == b->n_circ) {
+            if (!cb_replan_pairs(b, gates)) return cb_invalid("svb_cbatch_run: the plan's structure changed");
+            std::copy(gates, gates + b->gate_off[b->n_circ], b->gates.begin());
+            svb_status st = cb_run(b);
+            if (st != SVB_OK) return st;
+            if (energies) std::memcpy(energies, b->h_energy, b->n_circ * sizeof(double));
+            return SVB_OK;
+        }
         CbPlan plan;
         std::string err;
         if (!cb_build_plan(b, gates, b->tile_bits, b->use_pairs, plan, err)) return cb_invalid("svb_cbatch_run: " + err);

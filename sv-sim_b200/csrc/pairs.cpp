@@ -501,11 +501,10 @@ void write_block(PairPlan& plan, const Block& b, bool transposed)
 
 }  // namespace
 
-namespace {
-
 bool plan_pairs_cut(const std::vector<EOp>& ops, int n, PairPlan& plan, const std::vector<Mat4>* mats, int seeds)
 {
     plan = PairPlan{};
+    plan.seeds = seeds;
     if (n < PR_TILE_BITS) return false;
     for (const EOp& e : ops) {
         if (e.form == F_SRN) return false;      // only real-linear: not a matrix
@@ -709,6 +708,7 @@ bool plan_pairs_cut(const std::vector<EOp>& ops, int n, PairPlan& plan, const st
     return true;
 }
 
+namespace {
 
 // Cost of a plan in units of one block, from the kernel's measured shares (n = 30: a
 // lane/register exchange 0.49, a lane permutation 0.36, a relayout 2.05, a pass's tile

@@ -191,6 +191,7 @@ struct PairPlan {
     std::vector<double> gates;           // per variant: 32 lanes x (B0, B1)
     size_t n_blocks = 0, n_swaps = 0, n_relayouts = 0, n_lane_perms = 0;
     size_t stage_bytes = 0;              // largest per-pass copy into shared memory
+    int seeds = 1;                       // select_passes seeds of the cut it was made with
 };
 
 // 4x4 complex matrix of an F_M4 op, row-major, re/im interleaved (index a = bit0 + 2 bit1)
@@ -202,6 +203,9 @@ using Mat4 = std::array<double, 32>;
 // short circuit, such as the adjoint's forward segments, plan the program-order cut only).
 bool plan_pairs(const std::vector<EOp>& ops, int n, PairPlan& plan, const std::vector<Mat4>* mats = nullptr,
                 bool both_cuts = true);
+// The plan of one cut (PairPlan::seeds of an earlier plan of the same structure gives that
+// plan again with new angles, at half the planning time).
+bool plan_pairs_cut(const std::vector<EOp>& ops, int n, PairPlan& plan, const std::vector<Mat4>* mats, int seeds);
 
 struct DevPairBuffers {
     PairPass* passes = nullptr;
