@@ -382,26 +382,47 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qaoa(QaoaArgs A)
                 }
             }
             // stages 0..3: mixer on the owned bits, with exchanges between stages
+            // A pass whose bits from jb on begin above a stage's has nothing to do there and
+            // goes to the next owner at once: the exchange it spares costs more than the
+            // branch (problems of 10 to 22 qubits, 4 layers, with gradients: 192 in FP64
+            // 34.69 -> 34.32 ms, 512 in FP32 63.30 -> 61.88 ms).
+            constexpr int own2 = C::reg_bit(2, 0), own3 = C::reg_bit(3, 0);
             if (fwd) {
                 // the exchanges alternate between the two buffers (lambda's is free on the
                 // forward sweep), so a buffer is written again only after a barrier that
                 // every read of it precedes
                 stage_rx<T, 0, false>(ps, ls, jb, je, c, s, part_b);
-                exchange<T, 0, 1>(ps, bp, tb0, tb1);
-                stage_rx<T, 1, false>(ps, ls, jb, je, c, s, part_b);
-                exchange<T, 1, 2>(ps, bl, tb1, tb2);
-                stage_rx<T, 2, false>(ps, ls, jb, je, c, s, part_b);
-                exchange<T, 2, 3>(ps, bp, tb2, tb3);
+                if (jb >= own3) {
+                    exchange<T, 0, 3>(ps, bp, tb0, tb3);
+                } else {
+                    if (jb >= own2) {
+                        exchange<T, 0, 2>(ps, bl, tb0, tb2);
+                    } else {
+                        exchange<T, 0, 1>(ps, bp, tb0, tb1);
+                        stage_rx<T, 1, false>(ps, ls, jb, je, c, s, part_b);
+                        exchange<T, 1, 2>(ps, bl, tb1, tb2);
+                    }
+                    stage_rx<T, 2, false>(ps, ls, jb, je, c, s, part_b);
+                    exchange<T, 2, 3>(ps, bp, tb2, tb3);
+                }
                 stage_rx<T, 3, false>(ps, ls, jb, je, c, s, part_b);
             } else {
                 stage_rx<T, 0, true>(ps, ls, jb, je, c, s, part_b);
-                exchange2<T, 0, 1>(ps, ls, bp, bl, tb0, tb1);
-                stage_rx<T, 1, true>(ps, ls, jb, je, c, s, part_b);
-                __syncthreads();
-                exchange2<T, 1, 2>(ps, ls, bp, bl, tb1, tb2);
-                stage_rx<T, 2, true>(ps, ls, jb, je, c, s, part_b);
-                __syncthreads();
-                exchange2<T, 2, 3>(ps, ls, bp, bl, tb2, tb3);
+                if (jb >= own3) {
+                    exchange2<T, 0, 3>(ps, ls, bp, bl, tb0, tb3);
+                } else {
+                    if (jb >= own2) {
+                        exchange2<T, 0, 2>(ps, ls, bp, bl, tb0, tb2);
+                    } else {
+                        exchange2<T, 0, 1>(ps, ls, bp, bl, tb0, tb1);
+                        stage_rx<T, 1, true>(ps, ls, jb, je, c, s, part_b);
+                        __syncthreads();
+                        exchange2<T, 1, 2>(ps, ls, bp, bl, tb1, tb2);
+                    }
+                    stage_rx<T, 2, true>(ps, ls, jb, je, c, s, part_b);
+                    __syncthreads();
+                    exchange2<T, 2, 3>(ps, ls, bp, bl, tb2, tb3);
+                }
                 stage_rx<T, 3, true>(ps, ls, jb, je, c, s, part_b);
             }
             // stage 3: diagonal work on the final layout, then registers -> HBM

@@ -153,3 +153,30 @@ def test_sharded_wrapper_single_process_equals_batch():
     e1, g1 = sq.run(g, bt)
     sq.close()
     assert np.array_equal(e0, e1) and np.array_equal(g0, g1)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_mixer_angles_over_the_whole_circle(precision):
+    """beta where cos or sin vanish, at the line between the two forms of the mixer (pi / 4),
+    negative and beyond pi, at sizes on both sides of every line of the pass structure (one
+    tile; high passes that own 1 to 10 bits): energies and gradients against svb_adjoint."""
+    from svsim_b200 import _native as nat
+    rng = np.random.default_rng(8)
+    betas = [0.0, np.pi / 2, np.pi / 4, 3 * np.pi / 4, np.pi, -0.3, 1e-9, np.pi / 2 - 1e-9, 2.0, np.pi / 4 + 1e-12]
+    sizes = [4, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22]
+    insts = [circuits.qaoa_instances(1, n, n, 3, seed=n)[0] for n in sizes]
+    for i, inst in enumerate(insts):
+        inst.betas[:] = [betas[(3 * i + k) % len(betas)] for k in range(3)]
+        inst.gammas[:] = rng.uniform(-np.pi, np.pi, 3)
+    g, bt = params_of(insts)
+    e, grad = nat.QaoaBatch(insts, 0, precision).run(g, bt)
+    for i, inst in enumerate(insts):
+        pc = inst.param_circuit()
+        h = nat.Handle(inst.n, 0, nat.SVB_FP64)
+        want, wg = h.adjoint(pc.gates, pc.binding, len(pc.params), inst.maxcut_terms())
+        h.close()
+        scale = max(1.0, float(np.max(np.abs(wg))))
+        # FP64: sums of 2^n terms; FP32: the rounding of 6 passes of FP32 amplitudes
+        tol = 1e-11 if precision == 0 else 2e-4
+        assert abs(e[i] - want) <= tol * max(1.0, abs(want)), (inst.n, e[i], want)
+        assert np.max(np.abs(grad[i] - wg)) <= tol * scale, (inst.n, grad[i], wg)
