@@ -104,32 +104,29 @@ __device__ __forceinline__ double from_grid(uint32_t code, uint64_t m)   // m in
     return __longlong_as_double((long long)(((uint64_t)code << 52) | (m - HIDDEN)));
 }
 
-// p / 2^(e-52) rounded to the nearest integer, for p >= 0 (e = code - 1023).  *ok is
-// cleared on a tie (fraction exactly 1/2) and for NaN or inf.  Exact integer
-// arithmetic on p's significand.
-__device__ __forceinline__ uint64_t grid_units(double p, uint32_t code, bool* ok)
+// A binade's grid unit as two factors, p / 2^(e-52) = p * a * b with e = code - 1023 in
+// [-1022, 1023]: 2^(52-e) alone can lie outside the doubles.
+struct Grid { double a, b; };
+__device__ __forceinline__ Grid grid_of(uint32_t code)
 {
-    const uint64_t b = (uint64_t)__double_as_longlong(p);
-    const int pb = (int)((b >> 52) & 0x7ff);
-    if (pb == 0x7ff) { *ok = false; return 0; }
-    uint64_t mp = b & FRAC_MASK;
-    int ep = -1022;
-    if (pb != 0) { mp |= HIDDEN; ep = pb - 1023; }
-    const int sh = ((int)code - 1023) - ep;          // p / u = mp * 2^-sh
-    if (sh < 0) {                                    // p >= 2^53 u: leaves the binade
-        if (mp != 0) *ok = false;
-        return 0;
-    }
-    if (sh == 0) {                                   // p / u = mp
-        if (mp >= HIDDEN) *ok = false;
-        return mp;
-    }
-    if (sh >= 64) return 0;                          // p / u < 2^-11
-    const uint64_t ip = mp >> sh;
-    const uint64_t fr = mp & ((1ull << sh) - 1);
-    const uint64_t half = 1ull << (sh - 1);
-    if (fr == half) *ok = false;
-    return ip + (fr > half ? 1 : 0);
+    const int k = 52 + 1023 - (int)code, h = k >> 1;
+    return {__longlong_as_double((long long)(1023 + h) << 52), __longlong_as_double((long long)(1023 + k - h) << 52)};
+}
+
+// p / 2^(e-52) rounded to the nearest integer, for p >= 0.  *ok is cleared on a tie
+// (fraction exactly 1/2), where p alone leaves the binade (p / u >= 2^52), and for NaN or
+// inf; the result is then not used.  Both products are exact (or below 2^-900, rounded
+// to 0 units either way), x + 2^52 rounds to an integer, and x - round(x) is exact.  In
+// doubles without a branch: shifts of the significand took some fifty instructions in
+// five branches, which also kept a lane's loads from being in flight together.
+__device__ __forceinline__ uint64_t grid_units(double p, Grid g, bool* ok)
+{
+    constexpr double TWO52 = 4503599627370496.0;
+    const double x = __dmul_rn(__dmul_rn(p, g.a), g.b);
+    const double y = __dadd_rn(x, TWO52);
+    const double frac = __dadd_rn(x, -__dadd_rn(y, -TWO52));
+    if (!(x < TWO52) || fabs(frac) == 0.5) *ok = false;
+    return (uint64_t)(__double_as_longlong(y) - __double_as_longlong(TWO52));
 }
 
 // S advanced by `d` grid units of binade `code`, if S lies in that binade and stays
@@ -153,7 +150,7 @@ __device__ __forceinline__ double chunk_scan_exact(double s_in, double p, int la
     const uint32_t code = binade_of(s_in, &m);
     if (code != 0) {
         bool ok = true;
-        const uint64_t d = grid_units(p, code, &ok);
+        const uint64_t d = grid_units(p, grid_of(code), &ok);
         uint64_t incl = d;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -213,7 +210,7 @@ __device__ double walk_block(const typename VecOf<T>::type* __restrict__ sv, uin
                 for (int k = 0; k < CHUNKS * 32 / CHAIN_THREADS; k++) {
                     const int c = warp + k * (CHAIN_THREADS / 32);
                     bool ok = true;
-                    const uint64_t d = warp_sum_u64(grid_units(sm.p[c * 32 + lane], code, &ok));
+                    const uint64_t d = warp_sum_u64(grid_units(sm.p[c * 32 + lane], grid_of(code), &ok));
                     ok = __all_sync(0xffffffffu, ok);
                     if (lane == 0) {
                         sm.delta[c] = d;     // each unit is at most 2^53: no wrap
@@ -373,7 +370,7 @@ k_cdf_blocks(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint6
         for (int k = 0; k < 16; k++) {
             nonzero |= (p[k] != 0.0);
             nan_free &= (p[k] == p[k]);
-            if (code != 0) acc += grid_units(p[k], code, &ok);
+            if (code != 0) acc += grid_units(p[k], grid_of(code), &ok);
         }
         acc = warp_sum_u64(acc);               // 4096 terms of at most 2^52: no wrap
         if (lane == 0) red[tid >> 5] = acc;
@@ -547,10 +544,48 @@ k_cdf_fill(const uint64_t* __restrict__ entry, uint64_t nblocks, uint64_t nsuper
     }
 }
 
+// Grid units of 16 consecutive chunks on binade `code`'s grid: lanes 2c and 2c + 1 receive
+// chunk c's sum and whether it has no tie, NaN or inf.  The 16 loads a lane are in flight
+// together and the 16 sums share one exchange (31 shuffles a lane instead of 160).
+constexpr int SHOT_GROUP = 16;
+template <typename T>
+__device__ __forceinline__ uint64_t group_units(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim,
+                                                uint64_t first, uint32_t code, int lane, bool* fits)
+{
+    const Grid grid = grid_of(code);
+    double p[SHOT_GROUP];
+    uint64_t d[SHOT_GROUP];
+    uint32_t bad = 0;
+#pragma unroll
+    for (int c = 0; c < SHOT_GROUP; c++) p[c] = prob_at<T>(sv, dim, first + (uint64_t)c * 32 + lane);
+#pragma unroll
+    for (int c = 0; c < SHOT_GROUP; c++) {
+        bool ok = true;
+        d[c] = grid_units(p[c], grid, &ok);
+        if (!ok) bad |= 1u << c;
+    }
+    *fits = !(__reduce_or_sync(0xffffffffu, bad) >> (lane >> 1) & 1);
+#pragma unroll
+    for (int h = SHOT_GROUP / 2; h >= 1; h >>= 1) {
+        const bool up = lane & (2 * h);          // this lane keeps the upper half of its sums
+#pragma unroll
+        for (int k = 0; k < h; k++) {
+            const uint64_t mine = up ? d[k + h] : d[k], theirs = up ? d[k] : d[k + h];
+            d[k] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * h);
+        }
+    }
+    return d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+}
+
 // Pass 6: one warp per shot.  start[] holds the reference's S at every block start
 // (start[nblocks] = S_{2^n}); the block with start[b] <= r < start[b+1] is walked with
 // the exact chunk sums until the first index j whose S_{j+1} exceeds r, which is the
-// reference's j with S_j <= r < S_{j+1}.  Shots with no such j (r >= S_{2^n}, r < 0 or
+// reference's j with S_j <= r < S_{j+1}.  A group of 16 chunks is summed at once; its first
+// chunk that ties, leaves the binade or ends above r is added element by element, and only a
+// new binade forms the sums again.  Bound by the slowest shot's chain of groups and chunks,
+// which lies in block 0, where S crosses a binade or ties every few chunks: 1,024 shots took
+// 94 us while such a group was added element by element throughout, 34 us now (n = 16; 30 at
+// n = 23).  Shots with no such j (r >= S_{2^n}, r < 0 or
 // NaN) give 0 as in the reference.
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -573,51 +608,41 @@ k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uin
         const uint64_t base = lo * BLOCK_AMPS;
         double s = start[lo];
         result = ~0ull;                  // replaced below: start[lo+1] > r is met inside the block
-        int c0 = 0, c1 = CHUNKS;         // chunks still to look through one by one
-        // groups of 16 chunks, their 16 loads a lane in flight together (one chunk at a
-        // time, a shot waited for up to 128 loads in turn: 95 us for 1,024 shots): a group
-        // without ties that stays in S's binade and ends at or below r is stepped over, and
-        // in the first that ends above r its chunks' sums are looked through the same way
-        for (int g = 0; g < CHUNKS; g += 16) {
-            uint64_t m;
+        uint32_t have = 0;               // binade code and group that the sums are formed for
+        int group = -1;
+        uint64_t units = 0;              // grid units of chunk group + lane / 2, and its ties
+        bool fits = false;
+        for (int cur = 0; cur < CHUNKS && base + (uint64_t)cur * 32 < dim;) {
+            uint64_t m = 0;
             const uint32_t code = binade_of(s, &m);
-            c0 = g;
-            if (code == 0) break;
-            bool ok = true;
-            uint64_t d[16], sum = 0;
-#pragma unroll
-            for (int c = 0; c < 16; c++)
-                d[c] = grid_units(prob_at<T>(sv, dim, base + (uint64_t)(g + c) * 32 + lane), code, &ok);
-#pragma unroll
-            for (int c = 0; c < 16; c++) sum += d[c];
-            sum = warp_sum_u64(sum);     // 512 terms of at most 2^53: no wrap
-            if (!__all_sync(0xffffffffu, ok) || sum > M_MAX - m) break;
-            const double end = from_grid(code, m + sum);
-            if (end <= r) {
-                s = end;
-                c0 = CHUNKS;
-                continue;
-            }
-            uint64_t pre = 0;            // units of the chunks that end at or below r
-            int f = 0;
-            bool open = true;
-#pragma unroll
-            for (int c = 0; c < 16; c++) {
-                const uint64_t t = warp_sum_u64(d[c]);
-                open = open && from_grid(code, m + pre + t) <= r;
-                if (open) {
-                    pre += t;
-                    f = c + 1;
+            int f = cur;                 // chunk to add element by element
+            if (code != 0) {
+                const int g = cur & ~(SHOT_GROUP - 1);
+                if (code != have || g != group) {
+                    units = group_units<T>(sv, dim, base + (uint64_t)g * 32, code, lane, &fits);
+                    have = code;
+                    group = g;
                 }
+                const int c = g + (lane >> 1);
+                const bool in = !(lane & 1) && c >= cur;
+                const uint64_t v = in ? units : 0;
+                uint64_t incl = v;       // 16 sums of at most 2^58: no wrap
+#pragma unroll
+                for (int o = 2; o < 32; o <<= 1) {
+                    const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                const unsigned stop = __ballot_sync(
+                    0xffffffffu, in && (!fits || incl > M_MAX - m || from_grid(code, m + incl) > r));
+                const int l = stop ? __ffs(stop) - 1 : 30;
+                s = from_grid(code, m + __shfl_sync(0xffffffffu, stop ? incl - v : incl, l));
+                if (!stop) {
+                    cur = g + SHOT_GROUP;
+                    continue;
+                }
+                f = g + (l >> 1);
             }
-            s = from_grid(code, m + pre);
-            c0 = g + f;                  // f < 16: the group ends above r
-            c1 = c0 + 1;
-            break;
-        }
-        for (int c = c0; c < c1; c++) {
-            const uint64_t i0 = base + (uint64_t)c * 32;
-            if (i0 >= dim) break;
+            const uint64_t i0 = base + (uint64_t)f * 32;
             const double incl = chunk_scan_exact(s, prob_at<T>(sv, dim, i0 + lane), lane);
             const unsigned hit = __ballot_sync(0xffffffffu, incl > r);
             if (hit) {
@@ -625,6 +650,7 @@ k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uin
                 break;
             }
             s = __shfl_sync(0xffffffffu, incl, 31);
+            cur = f + 1;
         }
     }
     if (lane == 0) out[shot] = result;

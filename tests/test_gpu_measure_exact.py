@@ -166,3 +166,21 @@ def test_edges_around_the_walked_sizes(oracle, n, maker):
         st = maker(n, rng)
     h.set_state(st[0], st[1])
     check_state(oracle, h, n, rng)
+
+
+@pytest.mark.parametrize("scale", [1e-161, 1e-150, 1e-120, 1e120, 1e150, 3e153])
+def test_edges_at_the_ends_of_the_double_range(oracle, scale):
+    """The grid unit 2^(e-52) or its inverse is no double for the first and last of these, and
+    probabilities are subnormal (1e-161) or their sum overflows (3e153): the samples and the
+    total are still those of the sequential sums, bit for bit."""
+    nat = native()
+    rng = np.random.default_rng(17)
+    re, im = rng.standard_normal((2, 1 << 15)) * scale
+    h = nat.Handle(15, 0, nat.SVB_FP64)
+    h.set_state(re, im)
+    scan = sequential_scan(re, im)
+    u = np.concatenate([edge_uniforms(scan, rng)[:-512], rng.random(512) * min(scan[-1], 1e308)])
+    got, total = h.measure(u)
+    want, wtotal = oracle.measure(15, re, im, u)
+    assert np.array_equal(got, want)
+    assert total == wtotal == scan[-1]
