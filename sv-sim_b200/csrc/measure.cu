@@ -14,17 +14,19 @@
 // tie: round-half-even then depends on the last bit of m) or m + p/u reaches 2^53 (the
 // sum leaves the binade and the grid doubles).  So a run of elements without ties
 // that stays in the binade advances m by an exact integer sum of per-element
-// roundings, which adds up in any order.  Ties and binade crossings (at most a few
-// dozen crossings, S being non-decreasing) are added one element at a time with
-// IEEE adds in index order.
+// roundings, which adds up in any order.  After a tie m is even whatever it was, so a
+// run with ties depends on m's first parity alone: it is a pair (d for even m, d + t for
+// odd m, t = -1, 0 or 1) and runs join associatively (struct Run).  Binade crossings (at
+// most a few dozen, S being non-decreasing) are added one element at a time with IEEE
+// adds in index order.
 //
 // Passes (B = 4096 amplitudes per block, 64 blocks per superblock):
 //   1. k_block_sums   approximate FP64 block sums (any order) -> k_scan_single gives
 //                     an approximate prefix, used only to guess each block's binade;
-//   2. k_cdf_blocks   per block: the exact integer sum D_b of round(p_i/u) on the
-//                     guessed binade's grid, or "zero block" / "no delta" (a tie, a
-//                     guessed crossing, or no normal start);
-//   3. k_cdf_super    per superblock: the sum of its blocks' D_b when they share one
+//   2. k_cdf_blocks   per block: the exact run D_b of its round(p_i/u) on the guessed
+//                     binade's grid, or "zero block" / "no delta" (a guessed crossing,
+//                     or no normal start);
+//   3. k_cdf_super    per superblock: its blocks' D_b joined when they share one
 //                     binade, else "no delta";
 //   4. k_cdf_chain    one CTA walks the superblocks in order from S = 0: a delta
 //                     applies when S is in its binade and stays there (checked on the
@@ -53,15 +55,76 @@ constexpr uint64_t WALK_BLOCKS = 4;
 constexpr uint64_t FRAC_MASK = (1ull << 52) - 1;
 constexpr uint64_t HIDDEN = 1ull << 52;
 constexpr uint64_t M_MAX = (1ull << 53) - 1;       // largest grid count inside one binade
-// A block or superblock entry: bits 0..52 hold the delta D in grid units, bits 53..63
+// A block or superblock entry: bits 0..52 hold its run (d below DELTA_END), bits 53..63
 // the biased exponent code of its binade (e + 1023, in [1, 2046]); code 0 = no delta
-// (its D field is then 1 if no probability of the range is NaN), code 2047 = every
+// (the field is then 1 if no probability of the range is NaN), code 2047 = every
 // probability of the range is zero.
 constexpr uint32_t CODE_NONE = 0, CODE_ZERO = 2047;
 
 __device__ __forceinline__ uint64_t pack_entry(uint64_t d, uint32_t code) { return (uint64_t)code << 53 | d; }
 __device__ __forceinline__ uint32_t entry_code(uint64_t w) { return (uint32_t)(w >> 53); }
 __device__ __forceinline__ uint64_t entry_delta(uint64_t w) { return w & M_MAX; }
+constexpr uint64_t DELTA_END = ((1ull << 53) - 1) / 3;   // 3 d + t + 1 fits the field
+
+// Elements added in one binade: m advances by d if it is even, by d + t if it is odd.
+struct Run {
+    uint64_t d;
+    int t;
+};
+// A run in 64 bits (d up to 2^57: 32 elements below 2^52).
+__device__ __forceinline__ uint64_t pack_run(Run a) { return a.d << 2 | (uint64_t)(a.t + 1); }
+__device__ __forceinline__ Run unpack_run(uint64_t w) { return {w >> 2, (int)(w & 3) - 1}; }
+__device__ __forceinline__ uint64_t entry_field(Run a) { return a.d * 3 + (uint64_t)(a.t + 1); }
+__device__ __forceinline__ Run entry_run(uint64_t w)
+{
+    const uint64_t f = entry_delta(w), d = f / 3;
+    return {d, (int)(f - d * 3) - 1};
+}
+__device__ __forceinline__ Run join(Run a, Run b)  // a, then b
+{
+    const bool odd = a.d & 1;
+    return {a.d + b.d + (uint64_t)(int64_t)(odd ? b.t : 0), a.t ? a.t : (odd ? -b.t : b.t)};
+}
+__device__ __forceinline__ uint64_t units_from(uint64_t m, Run a) { return a.d + (uint64_t)(int64_t)((m & 1) ? a.t : 0); }
+
+// One element per lane joined in lane order.  m is even after a tie, so what a tie adds
+// depends on the odd elements between it and the tie before, which two ballots show: a lane
+// receives its own element's units for even m at lane 0 (their sum is the run's d), and *t
+// and *odd (the sum's parity) are the run's.
+__device__ __forceinline__ uint64_t warp_run(Run a, int lane, int* t, int* odd)
+{
+    const uint32_t ones = __ballot_sync(0xffffffffu, a.t == 0 && (a.d & 1));
+    const uint32_t ties = __ballot_sync(0xffffffffu, a.t != 0);
+    *t = 0;
+    *odd = __popc(ones) & 1;
+    if (ties == 0) return a.d;
+    const uint32_t lt = (1u << lane) - 1, before = ties & lt;
+    const uint32_t since = before ? lt & ~((2u << (31 - __clz(before))) - 1) : lt;
+    const bool from_odd = __popc(ones & since) & 1;
+    *t = __shfl_sync(0xffffffffu, from_odd ? -a.t : a.t, __ffs(ties) - 1);
+    *odd = __popc(ones & ~((2u << (31 - __clz(ties))) - 1)) & 1;
+    return a.d + (uint64_t)(int64_t)(from_odd ? a.t : 0);
+}
+
+// The runs of a warp's lanes joined in lane order; lane 0 has the result.
+__device__ __forceinline__ Run warp_join(Run a)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        a = join(a, unpack_run(__shfl_down_sync(0xffffffffu, pack_run(a), o)));
+    return a;
+}
+
+// Lane l: the runs of lanes 0..l joined.
+__device__ __forceinline__ Run warp_scan(Run a, int lane)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Run b = unpack_run(__shfl_up_sync(0xffffffffu, pack_run(a), o));
+        if (lane >= o) a = join(b, a);
+    }
+    return a;
+}
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -113,28 +176,39 @@ __device__ __forceinline__ Grid grid_of(uint32_t code)
     return {__longlong_as_double((long long)(1023 + h) << 52), __longlong_as_double((long long)(1023 + k - h) << 52)};
 }
 
-// p / 2^(e-52) rounded to the nearest integer, for p >= 0.  *ok is cleared on a tie
-// (fraction exactly 1/2), where p alone leaves the binade (p / u >= 2^52), and for NaN or
-// inf; the result is then not used.  Both products are exact (or below 2^-900, rounded
+// p / 2^(e-52) rounded to the nearest integer, for p >= 0, as a run (a tie goes to the even
+// integer, so an odd m takes one unit more where that was down and one less where it was
+// up).  *ok is cleared where p alone leaves the binade (p / u >= 2^52) and for NaN or inf;
+// the result is then not used.  Both products are exact (or below 2^-900, rounded
 // to 0 units either way), x + 2^52 rounds to an integer, and x - round(x) is exact.  In
 // doubles without a branch: shifts of the significand took some fifty instructions in
 // five branches, which also kept a lane's loads from being in flight together.
-__device__ __forceinline__ uint64_t grid_units(double p, Grid g, bool* ok)
+__device__ __forceinline__ Run grid_run(double p, Grid g, bool* ok)
 {
     constexpr double TWO52 = 4503599627370496.0;
     const double x = __dmul_rn(__dmul_rn(p, g.a), g.b);
     const double y = __dadd_rn(x, TWO52);
     const double frac = __dadd_rn(x, -__dadd_rn(y, -TWO52));
-    if (!(x < TWO52) || fabs(frac) == 0.5) *ok = false;
-    return (uint64_t)(__double_as_longlong(y) - __double_as_longlong(TWO52));
+    if (!(x < TWO52)) *ok = false;
+    return {(uint64_t)(__double_as_longlong(y) - __double_as_longlong(TWO52)),
+            frac == 0.5 ? 1 : frac == -0.5 ? -1 : 0};
 }
 
-// S advanced by `d` grid units of binade `code`, if S lies in that binade and stays
-// there; returns false (S unchanged) otherwise.
-__device__ __forceinline__ bool advance(double* s, uint32_t code, uint64_t d)
+// The same where a tie is not wanted: it clears *ok too.
+__device__ __forceinline__ uint64_t grid_units(double p, Grid g, bool* ok)
+{
+    const Run a = grid_run(p, g, ok);
+    if (a.t) *ok = false;
+    return a.d;
+}
+
+// S advanced by a run of binade `code`, if S lies in that binade and stays there; returns
+// false (S unchanged) otherwise.
+__device__ __forceinline__ bool advance(double* s, uint32_t code, Run a)
 {
     uint64_t m;
     if (binade_of(*s, &m) != code || code == 0) return false;
+    const uint64_t d = units_from(m, a);
     if (d > M_MAX - m) return false;
     *s = from_grid(code, m + d);
     return true;
@@ -173,19 +247,25 @@ __device__ __forceinline__ double chunk_scan_exact(double s_in, double p, int la
 
 // The chain's CTA.  Its 16 warps share one block's probabilities in shared memory; one warp
 // alone walked a block in 48-190 us (128 dependent chunk loads and scans), and a state has
-// a walked block per binade that S crosses, 12 to 25 of them.
+// a walked block per binade that S crosses, 12 to 25 of them.  Bound by that chain of
+// crossings, each a chunk's dependent adds and the deltas after it formed again.  The chain
+// of 2^16 / 2^23 amplitudes: 749 / 2,227 us with one warp, 91 / 299 with the CTA, 61 / 252
+// with the branch-free rounding, 54 / 137 since blocks with ties (one in b at block b, in a
+// state of even weight) have deltas and are not walked.
 constexpr int CHAIN_THREADS = 512;
 struct WalkSmem {
     double p[BLOCK_AMPS];
-    uint64_t delta[CHUNKS];          // a chunk's grid units in the current binade
-    uint32_t ok[CHUNKS];             // no tie, NaN or inf among them
+    uint64_t run[CHUNKS];            // a chunk's run in the current binade
+    uint32_t ok[CHUNKS];             // no NaN or inf in it, and none that leaves the binade alone
+    double s;                        // warp 0's sum and the chunks it has added
+    int cur;
 };
 
 // S after block b, exactly, from s at its start; every thread of the CTA calls it with the
-// same s and receives the same result.  The chunks' grid units are summed for the current
-// binade by all warps at once; a warp-wide scan over the 128 chunks (four a lane, the same
-// in every warp) finds the first chunk that ties or leaves the binade, that chunk is added
-// element by element, and the sums are formed again only when the binade changed.
+// same s and receives the same result.  The chunks' runs are formed for the current binade
+// by all warps at once; a warp-wide scan over the 128 chunks (four a lane, the same in every
+// warp) finds the first chunk that leaves the binade, that chunk is added element by
+// element, and the runs of the chunks after it are formed again for the new binade.
 template <typename T>
 __device__ double walk_block(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t b,
                              double s, WalkSmem& sm)
@@ -193,85 +273,93 @@ __device__ double walk_block(const typename VecOf<T>::type* __restrict__ sv, uin
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t base = b * BLOCK_AMPS;
     const int chunks = dim - base < BLOCK_AMPS ? (int)((dim - base + 31) / 32) : CHUNKS;
-    __syncthreads();                         // the previous block's readers are done
 #pragma unroll
     for (int k = 0; k < BLOCK_AMPS / CHAIN_THREADS; k++)
         sm.p[tid + k * CHAIN_THREADS] = prob_at<T>(sv, dim, base + tid + k * CHAIN_THREADS);
-    uint32_t have = 0;                       // binade code sm.delta is formed for
-    int cur = 0;
-    while (cur < chunks) {
+    __syncthreads();
+    for (int cur = 0; cur < chunks;) {
         uint64_t m = 0;
         const uint32_t code = binade_of(s, &m);
-        int f = cur;                         // chunk to add element by element
         if (code != 0) {
-            if (code != have) {
-                __syncthreads();             // sm.p is written; readers of the old sums are done
 #pragma unroll
-                for (int k = 0; k < CHUNKS * 32 / CHAIN_THREADS; k++) {
-                    const int c = warp + k * (CHAIN_THREADS / 32);
-                    bool ok = true;
-                    const uint64_t d = warp_sum_u64(grid_units(sm.p[c * 32 + lane], grid_of(code), &ok));
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (lane == 0) {
-                        sm.delta[c] = d;     // each unit is at most 2^53: no wrap
-                        sm.ok[c] = ok;
-                    }
+            for (int k = 0; k < CHUNKS * 32 / CHAIN_THREADS; k++) {
+                const int c = warp + k * (CHAIN_THREADS / 32);
+                if (c < cur) continue;
+                bool ok = true;
+                Run a = grid_run(sm.p[c * 32 + lane], grid_of(code), &ok);
+                ok = __all_sync(0xffffffffu, ok);
+                int odd;
+                a.d = warp_sum_u64(warp_run(a, lane, &a.t, &odd));
+                if (lane == 0) {
+                    sm.run[c] = pack_run(a);
+                    sm.ok[c] = ok;
                 }
-                __syncthreads();
-                have = code;
-            }
-            // inclusive sums of the chunks from cur on; a chunk with a tie ends the run.
-            // Sums are capped just above M_MAX so that 128 of them cannot wrap.
-            constexpr uint64_t OVER = 1ull << 54;
-            uint64_t v[4], run = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int c = lane * 4 + k;
-                const uint64_t d = (c < cur || c >= chunks) ? 0 : (sm.ok[c] && sm.delta[c] <= M_MAX ? sm.delta[c] : OVER);
-                run = run + d < OVER ? run + d : OVER;
-                v[k] = run;
-            }
-            uint64_t incl = run;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl = incl + y < OVER ? incl + y : OVER;
-            }
-            const uint64_t before = __shfl_up_sync(0xffffffffu, incl, 1);
-            const uint64_t excl = lane ? before : 0;
-            int bad = 4;                     // first of this lane's chunks that does not fit
-#pragma unroll
-            for (int k = 3; k >= 0; k--)
-                if (excl + v[k] > M_MAX - m) bad = k;
-            const unsigned who = __ballot_sync(0xffffffffu, bad < 4);
-            uint64_t pre = 0;                // grid units before chunk f
-            if (who) {
-                const int l = __ffs(who) - 1;
-                const uint64_t mine = excl + (bad == 0 || bad == 4 ? 0 : v[bad - 1]);
-                pre = __shfl_sync(0xffffffffu, mine, l);
-                f = l * 4 + __shfl_sync(0xffffffffu, bad, l);
-            } else {
-                pre = __shfl_sync(0xffffffffu, incl, 31);
-                f = chunks;
-            }
-            s = from_grid(code, m + pre);
-            if (f >= chunks) break;
-        } else {
-            if (s != s) break;               // NaN stays NaN
-            if (have == 0) {
-                __syncthreads();
-                have = ~0u;                  // sm.p is written; no sums formed
-            }
-            if (s == 0.0 && __all_sync(0xffffffffu, sm.p[f * 32 + lane] == 0.0)) {
-                cur = f + 1;
-                continue;
             }
         }
-        double x = s;
+        __syncthreads();                 // sm.run is written; sm.s has been read by all
+        // one warp goes on until the binade changes: in all sixteen the scan took four times
+        // as many issue slots
+        if (warp == 0) {
+            do {
+                int f = cur;                 // chunk to add element by element
+                if (code != 0) {
+                    // inclusive runs of the chunks from cur on.  They are capped just above M_MAX, as
+                    // is a chunk that is not ok, so that 128 of them cannot wrap.
+                    constexpr uint64_t OVER = 1ull << 54;
+                    Run v[4], run = {0, 0};
 #pragma unroll
-        for (int k = 0; k < 32; k++) x = __dadd_rn(x, sm.p[f * 32 + k]);
-        s = x;
-        cur = f + 1;
+                    for (int k = 0; k < 4; k++) {
+                        const int c = lane * 4 + k;
+                        Run a = {0, 0};
+                        if (c >= cur && c < chunks) a = sm.ok[c] ? unpack_run(sm.run[c]) : Run{OVER, 0};
+                        run = join(run, a);
+                        if (run.d > OVER) run.d = OVER;
+                        v[k] = run;
+                    }
+                    const Run incl = warp_scan(run, lane);   // up to 32 times OVER
+                    Run excl = unpack_run(__shfl_up_sync(0xffffffffu, pack_run(incl), 1));
+                    if (lane == 0) excl = {0, 0};
+                    int bad = 4;                     // first of this lane's chunks that does not fit
+                    uint64_t mine = units_from(m, excl);     // grid units before it
+#pragma unroll
+                    for (int k = 3; k >= 0; k--)
+                        if (units_from(m, join(excl, v[k])) > M_MAX - m) bad = k;
+#pragma unroll
+                    for (int k = 0; k < 3; k++)
+                        if (bad == k + 1) mine = units_from(m, join(excl, v[k]));
+                    const unsigned who = __ballot_sync(0xffffffffu, bad < 4);
+                    uint64_t pre = 0;                // grid units before chunk f
+                    if (who) {
+                        const int l = __ffs(who) - 1;
+                        pre = __shfl_sync(0xffffffffu, mine, l);
+                        f = l * 4 + __shfl_sync(0xffffffffu, bad, l);
+                    } else {
+                        pre = __shfl_sync(0xffffffffu, units_from(m, incl), 31);
+                        f = chunks;
+                    }
+                    s = from_grid(code, m + pre);
+                    if (f >= chunks) {
+                        cur = chunks;
+                        break;
+                    }
+                } else if (s != s) {         // NaN stays NaN
+                    cur = chunks;
+                    break;
+                }
+                if (code != 0 || !(s == 0.0 && __all_sync(0xffffffffu, sm.p[f * 32 + lane] == 0.0))) {
+#pragma unroll
+                    for (int k = 0; k < 32; k++) s = __dadd_rn(s, sm.p[f * 32 + k]);
+                }
+                cur = f + 1;
+            } while (cur < chunks && binade_of(s, &m) == code);
+            if (lane == 0) {
+                sm.s = s;
+                sm.cur = cur;
+            }
+        }
+        __syncthreads();
+        s = sm.s;
+        cur = sm.cur;
     }
     return s;
 }
@@ -354,37 +442,83 @@ k_cdf_blocks(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint6
              const double* __restrict__ approx, uint64_t* __restrict__ entry)
 {
     __shared__ uint64_t red[8];
-    const int tid = threadIdx.x, lane = tid & 31;
+    __shared__ uint32_t redf[8];
+    __shared__ uint64_t runs[CHUNKS], redt[8];
+    constexpr uint32_t NONZERO = 1, NAN_SEEN = 2, NOT_OK = 4, TIE = 8;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint64_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
         uint64_t m0, m1;
         const uint32_t c0 = binade_of(approx[b], &m0);
         const uint32_t c1 = binade_of(approx[b + 1], &m1);
         const uint32_t code = (c0 != 0 && c0 == c1) ? c0 : 0;
+        const Grid grid = grid_of(code);
         const uint64_t base = b * BLOCK_AMPS + tid;
         double p[16];
 #pragma unroll
         for (int k = 0; k < 16; k++) p[k] = prob_at<T>(sv, dim, base + k * 256);
         uint64_t acc = 0;
-        bool ok = true, nonzero = false, nan_free = true;
+        uint32_t flags = 0;
 #pragma unroll
         for (int k = 0; k < 16; k++) {
-            nonzero |= (p[k] != 0.0);
-            nan_free &= (p[k] == p[k]);
-            if (code != 0) acc += grid_units(p[k], grid_of(code), &ok);
+            bool ok = true;
+            const Run a = grid_run(p[k], grid, &ok);
+            acc += a.d;
+            flags |= (p[k] != 0.0 ? NONZERO : 0) | (p[k] != p[k] ? NAN_SEEN : 0) | (ok ? 0 : NOT_OK) | (a.t ? TIE : 0);
         }
         acc = warp_sum_u64(acc);               // 4096 terms of at most 2^52: no wrap
-        if (lane == 0) red[tid >> 5] = acc;
-        // the barriers below also order red[] before its readers and the next block's writers
-        nonzero = __syncthreads_or(nonzero);
-        nan_free = __syncthreads_and(nan_free);
-        ok = __syncthreads_and(ok);
-        if (tid == 0) {
+        flags = __reduce_or_sync(0xffffffffu, flags);
+        if (lane == 0) {
+            red[warp] = acc;
+            redf[warp] = flags;
+        }
+        __syncthreads();
+        flags = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) flags |= redf[w];
+        const bool use = code != 0 && !(flags & NOT_OK);
+        if (use && (flags & TIE)) {
+            // in index order: each chunk with its first m even, then the chunks' parities and
+            // what their first ties add for odd m, by one warp
+            uint64_t more = 0;                 // modulo 2^64: -1 or 1 a tie
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                bool ok = true;
+                int t, odd;
+                const Run a = grid_run(p[k], grid, &ok);
+                more += warp_run(a, lane, &t, &odd) - a.d;
+                if (lane == 0) runs[k * 8 + warp] = pack_run({(uint64_t)odd, t});
+            }
+            more = warp_sum_u64(more);
+            if (lane == 0) redt[warp] = red[warp] + more;
+            __syncthreads();
+            if (warp == 0) {
+                Run a = {0, 0};
+                uint64_t odds = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const Run c = unpack_run(runs[lane * 4 + k]);
+                    a = k ? join(a, c) : c;
+                    odds += c.d;
+                }
+                // a joined run of parities can be negative by its ties: an offset per lane
+                // that is even keeps it packable and no parity changes
+                a.d += 8;
+                a = warp_join(a);
+                odds = warp_sum_u64(odds) + 8 * 32;
+                if (lane == 0) {
+                    uint64_t sum = a.d - odds;
+#pragma unroll
+                    for (int w = 0; w < 8; w++) sum += redt[w];
+                    entry[b] = sum < DELTA_END ? pack_entry(entry_field({sum, a.t}), code) : pack_entry(1, CODE_NONE);
+                }
+            }
+        } else if (tid == 0) {
             acc = 0;
 #pragma unroll
             for (int w = 0; w < 8; w++) acc += red[w];
-            uint64_t w = pack_entry(nan_free ? 1 : 0, CODE_NONE);
-            if (!nonzero) w = pack_entry(0, CODE_ZERO);
-            else if (code != 0 && ok && acc < HIDDEN) w = pack_entry(acc, code);
+            uint64_t w = pack_entry(flags & NAN_SEEN ? 0 : 1, CODE_NONE);
+            if (!(flags & NONZERO)) w = pack_entry(0, CODE_ZERO);
+            else if (use && acc < DELTA_END) w = pack_entry(entry_field({acc, 0}), code);
             entry[b] = w;
         }
         __syncthreads();
@@ -401,7 +535,7 @@ k_cdf_super(const uint64_t* __restrict__ entry, uint64_t nblocks, uint64_t nsupe
     const uint64_t b0 = s * SUPER_BLOCKS;
     const uint64_t b1 = b0 + SUPER_BLOCKS < nblocks ? b0 + SUPER_BLOCKS : nblocks;
     uint32_t code = CODE_ZERO;
-    uint64_t d = 0;
+    Run d = {0, 0};
     bool ok = true, nan_free = true;
     for (uint64_t b = b0; b < b1; b++) {
         const uint64_t w = entry[b];
@@ -414,10 +548,10 @@ k_cdf_super(const uint64_t* __restrict__ entry, uint64_t nblocks, uint64_t nsupe
         }
         if (code != CODE_ZERO && c != code) ok = false;
         code = c;
-        d += entry_delta(w);                   // each < 2^52, at most 64 of them
-        if (d >= HIDDEN) ok = false;
+        d = join(d, entry_run(w));   // each below 2^52, at most 64 of them
+        if (d.d >= DELTA_END) ok = false;
     }
-    sentry[s] = ok ? pack_entry(code == CODE_ZERO ? 0 : d, code) : pack_entry(nan_free ? 1 : 0, CODE_NONE);
+    sentry[s] = ok ? pack_entry(code == CODE_ZERO ? 0 : entry_field(d), code) : pack_entry(nan_free ? 1 : 0, CODE_NONE);
 }
 
 // S can no longer change over a range: S is NaN, or S is +inf and no probability of
@@ -428,35 +562,35 @@ __device__ __forceinline__ bool stuck(double s, uint64_t w)
     return isinf(s) && (entry_code(w) != CODE_NONE || entry_delta(w) == 1);
 }
 
-// S over 32 consecutive superblocks (or blocks) at once: lane l holds entry w of the l-th of
-// them (cnt in all).  When every entry is zero or a delta of S's binade and S stays in the
-// binade, *s is advanced past all of them and *excl receives S at this lane's start.
-__device__ __forceinline__ bool advance_32(double* s, uint64_t w, uint64_t cnt, int lane, double* excl)
+// S over consecutive superblocks (or blocks), up to 32 at once: lane l holds entry w of the
+// l-th of them, and lanes from..cnt-1 are to be added.  Returns the first that S cannot be
+// advanced past (a delta of another binade or none, or S leaves the binade), or cnt; *s is
+// then S at its start, and *excl S at this lane's start for lanes from..that one.
+__device__ __forceinline__ int advance_32(double* s, uint64_t w, int from, int cnt, int lane, double* excl)
 {
-    uint64_t m;
-    const uint32_t code = binade_of(*s, &m);
-    if (code == 0) return false;
-    const uint32_t c = entry_code(w);
-    const bool in = (uint64_t)lane < cnt;
-    if (!__all_sync(0xffffffffu, !in || c == CODE_ZERO || c == code)) return false;
-    const uint64_t d = (in && c == code) ? entry_delta(w) : 0;     // each < 2^52
-    uint64_t incl = d;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+    uint64_t m = 0;
+    const uint32_t code = binade_of(*s, &m), c = entry_code(w);
+    const bool in = lane >= from && lane < cnt;
+    if (code == 0) {                         // zeros change no S
+        const unsigned stop = __ballot_sync(0xffffffffu, in && c != CODE_ZERO);
+        *excl = *s;
+        return stop ? __ffs(stop) - 1 : cnt;
     }
-    const uint64_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total > M_MAX - m) return false;
-    *excl = from_grid(code, m + (incl - d));
-    *s = from_grid(code, m + total);
-    return true;
+    const Run a = in && c == code ? entry_run(w) : Run{0, 0};
+    const uint64_t d = units_from(m, warp_scan(a, lane));    // up to 32 below 2^52
+    const uint64_t up = __shfl_up_sync(0xffffffffu, d, 1);
+    const uint64_t before = lane ? up : 0;
+    const unsigned stop = __ballot_sync(0xffffffffu, in && ((c != CODE_ZERO && c != code) || d > M_MAX - m));
+    const int f = stop ? __ffs(stop) - 1 : cnt;
+    *excl = from_grid(code, m + before);
+    *s = from_grid(code, m + __shfl_sync(0xffffffffu, stop ? before : d, stop ? f : 31));
+    return f;
 }
 
 // Pass 4: one CTA; every warp follows the same chain (S and the entries are the same in
 // all), warp 0 writes it down, and all of them share the work of a walked block.  Entries
-// are read 32 at a time (one per lane) and, where they are all deltas of S's binade, added
-// by one scan; else one by one.  desc[s] = 1 marks a superblock whose block starts the
+// are read 32 at a time (one per lane) and added by one scan up to the first that does not
+// apply, which is descended into.  desc[s] = 1 marks a superblock whose block starts the
 // chain wrote itself.  entry == nullptr: no deltas, every block is walked.
 template <typename T>
 __global__ void __launch_bounds__(CHAIN_THREADS)
@@ -478,42 +612,36 @@ k_cdf_chain(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64
     }
     for (uint64_t g = 0; g < nsuper; g += 32) {
         const uint64_t mine = g + lane < nsuper ? sentry[g + lane] : 0;
-        const uint64_t cnt = nsuper - g < 32 ? nsuper - g : 32;
-        if (advance_32(&s_val, mine, cnt, lane, &at)) {
-            if (wwarp && (uint64_t)lane < cnt) {
+        const int cnt = nsuper - g < 32 ? (int)(nsuper - g) : 32;
+        for (int k = 0; k < cnt; k++) {
+            const int from = k;
+            k = advance_32(&s_val, mine, from, cnt, lane, &at);
+            if (wwarp && lane >= from && lane < k) {
                 sstart[g + lane] = at;
                 desc[g + lane] = 0;
             }
-            continue;
-        }
-        for (uint64_t k = 0; k < cnt; k++) {
+            if (k == cnt) break;
             const uint64_t sidx = g + k;
-            const uint64_t w = __shfl_sync(0xffffffffu, mine, (int)k);
-            if (writer) sstart[sidx] = s_val;
-            const uint32_t code = entry_code(w);
-            if (code == CODE_ZERO || stuck(s_val, w) ||
-                (code != CODE_NONE && advance(&s_val, code, entry_delta(w)))) {
-                if (writer) desc[sidx] = 0;
-                continue;
+            const uint64_t w = __shfl_sync(0xffffffffu, mine, k);
+            const bool skip = stuck(s_val, w);
+            if (writer) {
+                sstart[sidx] = s_val;
+                desc[sidx] = !skip;
             }
-            if (writer) desc[sidx] = 1;
+            if (skip) continue;
             const uint64_t b0 = sidx * SUPER_BLOCKS;
             const uint64_t b1 = b0 + SUPER_BLOCKS < nblocks ? b0 + SUPER_BLOCKS : nblocks;
             for (uint64_t h = b0; h < b1; h += 32) {
                 const uint64_t bm = h + lane < b1 ? entry[h + lane] : 0;
-                const uint64_t bc = b1 - h < 32 ? b1 - h : 32;
-                if (advance_32(&s_val, bm, bc, lane, &at)) {
-                    if (wwarp && (uint64_t)lane < bc) start[h + lane] = at;
-                    continue;
-                }
-                for (uint64_t j = 0; j < bc; j++) {
-                    const uint64_t b = h + j;
-                    const uint64_t wb = __shfl_sync(0xffffffffu, bm, (int)j);
-                    if (writer) start[b] = s_val;
-                    const uint32_t cb = entry_code(wb);
-                    if (cb == CODE_ZERO || stuck(s_val, wb)) continue;
-                    if (cb != CODE_NONE && advance(&s_val, cb, entry_delta(wb))) continue;
-                    s_val = walk_block<T>(sv, dim, b, s_val, sm);
+                const int bc = b1 - h < 32 ? (int)(b1 - h) : 32;
+                for (int j = 0; j < bc; j++) {
+                    const int first = j;
+                    j = advance_32(&s_val, bm, first, bc, lane, &at);
+                    if (wwarp && lane >= first && lane < j) start[h + lane] = at;
+                    if (j == bc) break;
+                    if (writer) start[h + j] = s_val;
+                    if (!stuck(s_val, __shfl_sync(0xffffffffu, bm, j)))
+                        s_val = walk_block<T>(sv, dim, h + j, s_val, sm);
                 }
             }
         }
@@ -540,7 +668,7 @@ k_cdf_fill(const uint64_t* __restrict__ entry, uint64_t nblocks, uint64_t nsuper
         start[b] = v;
         const uint64_t w = entry[b];
         const uint32_t c = entry_code(w);
-        if (c != CODE_ZERO && c != CODE_NONE && v == v) advance(&v, c, entry_delta(w));
+        if (c != CODE_ZERO && c != CODE_NONE && v == v) advance(&v, c, entry_run(w));
     }
 }
 

@@ -184,3 +184,25 @@ def test_edges_at_the_ends_of_the_double_range(oracle, scale):
     want, wtotal = oracle.measure(15, re, im, u)
     assert np.array_equal(got, want)
     assert total == wtotal == scan[-1]
+
+
+@pytest.mark.parametrize("n", [14, 15, 17, 20])
+@pytest.mark.parametrize("share", [0.001, 0.5])
+def test_edges_with_ties_of_both_parities(oracle, n, share):
+    """Ties that round up and ties that round down, met with odd and with even grid counts, in
+    lanes, chunks, blocks and superblocks beside non-ties of odd units: S stays in [0.5, 1),
+    whose grid unit is 2^-53, and p is k or k + 1/2 units exactly."""
+    rng = np.random.default_rng(4000 + n)
+    units = np.arange(1, 40) * 0.5
+    amp = np.sqrt(units * 2.0 ** -53)
+    held = amp * amp == units * 2.0 ** -53          # survives the square as it is rounded
+    whole, half = amp[held & (units % 1 == 0)], amp[held & (units % 1 == 0.5)]
+    down = units[held & (units % 1 == 0.5)] // 1 % 2 == 0
+    assert down.any() and not down.all() and np.any(units[held & (units % 1 == 0)] % 2 == 1)
+    re = np.where(rng.random(1 << n) < share, rng.choice(half, 1 << n), rng.choice(whole, 1 << n))
+    re[0] = 0.75
+    im = np.zeros(1 << n)
+    nat = native()
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    h.set_state(re, im)
+    check_state(oracle, h, n, rng)
