@@ -600,10 +600,9 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     s->info.engine = engine;
     // the butterfly form of the pair engine (FP64) and, where no fusion width is asked for, of
     // the fused engine (FP32), for the circuits it is faster on
+    BfPlan B;
     if ((engine == SVB_ENGINE_PAIRS || (engine == SVB_ENGINE_FUSED && fusion == 0)) &&
-        bfly_preferred(s->eops, n, s->precision)) {
-        BfPlan B;
-        plan_bfly(s->eops, n, s->precision, B, true);
+        bfly_preferred(s->eops, n, s->precision) && plan_bfly(s->eops, n, s->precision, B, true)) {
         // an earlier circuit's kernels may still read the buffer, on any stream
         SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
         SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly), "plan upload");

@@ -260,6 +260,7 @@ struct PassPlanner {
     int op_limit = 0;                    // of plan.ops, where the pass has to end
     size_t coef_limit = 0;               // of plan.coefs
     const int32_t* stage_masks = nullptr; // tile masks of the pass's finished stages
+    bool ok = true;                      // false: a layout that the kernel cannot address
 
     int reg_of(const St& s, int p) const { return (pack && p == 0) ? BF_PACK : s.reg[p]; }
 
@@ -371,6 +372,10 @@ struct PassPlanner {
         if (i >= 0) {
             const uint8_t m = s.row[c].rm;
             if ((m >> i) & 1) return false;
+            // a position other than 0 cannot differ between the halves of a packed unit: its
+            // relayout slots and offsets are the unit's.  Registers that other rows share
+            // with t would make theirs differ; the next stage begins with pure rows.
+            if (pack && i != BF_PACK && ((m >> BF_PACK) & 1) && !column_pure(s, t)) return false;
             if (m) move_regs(s, t, m, dry);
         } else {
             if (pack && ((s.row[c].rm >> BF_PACK) & 1)) return false;
@@ -742,6 +747,7 @@ struct PassPlanner {
         out.clear();
         uint32_t wcol[BF_TB] = {0}, wreg[BF_RB] = {0};
         for (int x = pack; x < M; x++) {
+            if (s.row[x].rm >> BF_RB) ok = false;    // differs between the halves of a unit
             for (int b = 0; b < BF_TB; b++)
                 if ((s.row[x].tm >> bits[b]) & 1) wcol[b] |= 1u << x;
             for (int i = 0; i < BF_RB; i++)
@@ -914,7 +920,7 @@ std::vector<float> bfly_coefs32(const BfPlan& plan)
     return f;
 }
 
-void plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, bool tune)
+bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, bool tune)
 {
     plan = BfPlan{};
     const bool fp32 = precision == SVB_FP32;
@@ -984,8 +990,12 @@ void plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, 
         std::vector<const Item*> todo;
         for (int i : cuts[ci].second) todo.push_back(&items[i]);
         for (const Item& it : ends) todo.push_back(&it);
-        while (!todo.empty()) todo = pp.run(L, todo, cls);
+        while (!todo.empty()) {
+            todo = pp.run(L, todo, cls);
+            if (!pp.ok) return false;
+        }
     }
+    return true;
 }
 
 }  // namespace svb

@@ -768,7 +768,7 @@ extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, i
         if (!lower_gate(gates[i], (int32_t)i, eops)) return -1;
     if (!bfly_supported(eops, (int)n, precision)) return -5;
     BfPlan plan;
-    plan_bfly(eops, (int)n, precision, plan, tune != 0);
+    if (!plan_bfly(eops, (int)n, precision, plan, tune != 0)) return -8;
     stats[0] = plan.passes.size();
     stats[1] = plan.n_gates2;
     stats[2] = plan.n_diags;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from svsim_b200 import circuits, gates as G
-from test_plan import phase_circuit
+from test_plan import phase_circuit, shared_register
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +96,22 @@ def test_routes(oracle):
     re, im = h.get_state()
     want = oracle.run(16, np.concatenate([qft(16, 2), qft(16, 3)]))
     assert np.max(np.abs(re - want[0])) < 1e-13 and np.max(np.abs(im - want[1])) < 1e-13
+
+
+@pytest.mark.parametrize("n,t,y", [(13, 5, 2), (14, 9, 4), (16, 5, 2)])
+def test_packed_control_onto_a_shared_register(oracle, n, t, y):
+    """FP32, as the default dispatch runs it: a CX from qubit 0 onto a qubit whose register
+    another one depends on.  The circuits move and negate amplitudes: FP32 rounding of the
+    state only."""
+    from svsim_b200 import _native as nat
+    g = shared_register(n, t, y, 8)
+    st = np.random.default_rng(n).standard_normal((2, 1 << n))
+    st /= np.sqrt((st ** 2).sum())
+    h = nat.Handle(n, 0, nat.SVB_FP32)
+    h.set_circuit(g)
+    assert h.plan_info().n_blocks == 0
+    h.set_state(st[0], st[1])
+    h.run()
+    re, im = h.get_state()
+    want = oracle.run(n, g, state=(st[0], st[1]))
+    assert np.sqrt(np.sum((re - want[0]) ** 2 + (im - want[1]) ** 2)) <= 1.2e-7

@@ -477,3 +477,55 @@ def test_butterfly_plan_at_degenerate_angles(emu, oracle, theta, precision):
     want = oracle.run(n, g, state=(st[0], st[1]))
     err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
     assert rc == 0 and err <= 8 * (2.2e-16 if precision == 0 else 1.2e-7) * 10
+
+
+def shared_register(n, t, y, phases):
+    """CX(t -> y), after which y depends on t's register where y sits on a thread bit, then a CX
+    from qubit 0, which FP32 packs two to a unit, onto t."""
+    gl = [G.CX(t, y), G.CX(0, t)]
+    return G.to_array(gl + [G.CZ(q, (q + 3) % n) for q in range(phases)])
+
+
+@pytest.mark.parametrize("phases", [0, 8])
+@pytest.mark.parametrize("n,t,y", [(13, 5, 2), (14, 9, 4), (16, 5, 2)])
+def test_butterfly_plan_packed_control_onto_a_shared_register(emu, oracle, n, t, y, phases):
+    """A packed control's CX waits for the next stage where another row shares the target's
+    register: a row beside the packed one that differs between the halves of a unit has no
+    address.  FP32 rounding only (the circuits move amplitudes and negate them)."""
+    g = shared_register(n, t, y, phases)
+    for tune in (0, 1):
+        rc, got, st, _ = run_bfly(emu, n, g, 1, tune)
+        want = oracle.run(n, g, state=(st[0], st[1]))
+        err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+        assert rc == 0 and err <= 1.2e-7
+
+
+def short_circuit(n, rng):
+    """A few gates of every kind the planner treats differently, on qubit 0 more than on others."""
+    weights = ([4, 4, 0, 0, 0, 0, 0], [3, 1, 3, 2, 0, 0, 1], [4, 1, 1, 2, 2, 1, 1], [3, 0, 0, 1, 3, 1, 1])
+    w = np.array(weights[int(rng.integers(4))], dtype=float)
+    q = [0, 0] + list(range(n))
+    gl = []
+    for _ in range(int(2 ** rng.uniform(1, 6))):
+        a = int(rng.choice(q))
+        b = int(rng.choice([x for x in q if x != a]))
+        t = float(rng.uniform(-3, 3))
+        gl.append([lambda: G.CX(a, b), lambda: G.CZ(a, b), lambda: G.SWAP(a, b), lambda: G.H(a),
+                   lambda: G.U3(*rng.uniform(0, 6, 3), a), lambda: G.CU1(t, a, b),
+                   lambda: G.RX(t, a)][int(rng.choice(7, p=w / w.sum()))]())
+    return G.to_array(gl)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_butterfly_plan_on_random_short_circuits(emu, oracle, precision):
+    """300 seeded circuits of a precision: few gates, so that what one stage leaves to the next
+    differs from circuit to circuit."""
+    eps = 2.2e-16 if precision == 0 else 1.2e-7
+    for seed in range(300):
+        rng = np.random.default_rng(seed)
+        n = int(rng.integers(12, 15)) + precision
+        g = short_circuit(n, rng)
+        rc, got, st, _ = run_bfly(emu, n, g, precision, tune=seed & 1, seed=seed)
+        want = oracle.run(n, g, state=(st[0], st[1]))
+        err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+        assert rc == 0 and err <= 8 * eps * np.sqrt(100), (seed, rc, err)
