@@ -955,15 +955,15 @@ bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, 
         },
         tune ? 32 : 1);
     // the next cut that touches each qubit, from the last one backwards
-    std::vector<std::array<int16_t, 64>> next(cuts.size());
+    std::vector<std::array<int32_t, 64>> next(cuts.size());
     {
-        std::array<int16_t, 64> at;
+        std::array<int32_t, 64> at;
         at.fill(-1);
         for (size_t ci = cuts.size(); ci-- > 0;) {
             next[ci] = at;
             for (int i : cuts[ci].second)
                 for (int q = 0; q < n; q++)
-                    if ((items[i].touch >> q) & 1) at[q] = (int16_t)ci;
+                    if ((items[i].touch >> q) & 1) at[q] = (int32_t)ci;
         }
     }
     std::vector<M2> pend(64, ident2());
@@ -991,8 +991,9 @@ bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, 
         for (int i : cuts[ci].second) todo.push_back(&items[i]);
         for (const Item& it : ends) todo.push_back(&it);
         while (!todo.empty()) {
+            const size_t before = todo.size(), done = plan.n_gates2 + plan.n_diags + plan.n_moves;
             todo = pp.run(L, todo, cls);
-            if (!pp.ok) return false;
+            if (!pp.ok || (todo.size() == before && plan.n_gates2 + plan.n_diags + plan.n_moves == done)) return false;
         }
     }
     return true;

@@ -128,8 +128,8 @@ bool bfly_supported(const std::vector<EOp>& ops, int n, int precision);
 // bfly_supported.
 bool bfly_preferred(const std::vector<EOp>& ops, int n, int precision);
 // `tune` spends more host time on the choice of register qubits (1.5-3x the planning time).
-// False if a layout came out that the kernel cannot address (never seen; the caller then
-// takes another engine).
+// False if a layout came out that the kernel cannot address, or a pass that does nothing of
+// what is left (neither has been seen; the caller then takes another engine).
 bool plan_bfly(const std::vector<EOp>& ops, int n, int precision, BfPlan& plan, bool tune);
 
 // The coefficients as the kernel of FP32 states reads them.

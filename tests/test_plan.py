@@ -529,3 +529,20 @@ def test_butterfly_plan_on_random_short_circuits(emu, oracle, precision):
         want = oracle.run(n, g, state=(st[0], st[1]))
         err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
         assert rc == 0 and err <= 8 * eps * np.sqrt(100), (seed, rc, err)
+
+
+def test_butterfly_plan_of_a_circuit_with_many_cuts(emu):
+    """More than 32,767 passes: a period adds its own passes and gates and nothing else, so no
+    cut takes a later one for the last that touches a qubit (which would apply what is pending,
+    a phase a qubit)."""
+    n = 13
+    one = G.to_array([G.U3(0.3 + q, 0.2, 0.1, q) for q in range(n)] + [G.CX(q, (q + 1) % n) for q in range(n)])
+    stats = {}
+    for reps in (100, 200, 31000):
+        g = np.tile(one, reps)
+        st = (ctypes.c_uint64 * 8)()
+        assert emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), 0, 0, 0, None, None, st) == 0
+        stats[reps] = np.array([int(x) for x in st])
+    period = stats[200] - stats[100]
+    assert stats[31000][0] > 32767
+    assert np.array_equal((stats[31000] - stats[100])[:4] * 100, period[:4] * 30900), stats
