@@ -314,6 +314,8 @@ struct PassPlanner {
         }
     }
 
+    double round_to(double x) const { return fp32 ? (double)(float)x : x; }
+
     // applies what of pend[q] does not commute with a control (x = false) or target (x = true)
     void rot(St& s, int q, bool x, bool dry)
     {
@@ -325,16 +327,19 @@ struct PassPlanner {
         BfOp o = blank(BF_ROT);
         o.tgt = (uint8_t)reg_of(s, p);
         if (o.tgt == BF_PACK) o.kind = BF_PROT;
-        // the unscaled form grows amplitudes by 1/p: beyond these bounds (far inside the
-        // exponent range, and seldom met) the scale stays in the matrix
-        const double small = fp32 ? 1e-3 : 1e-6, least = fp32 ? 1e-24 : 1e-90;
         cplx u = sp.p > 0 ? sp.b / sp.p : cplx(0);
         const double ur = fp32 ? (float)u.real() : (double)u.real(), ui = fp32 ? (float)u.imag() : (double)u.imag();
         const real f = 1 / std::sqrt(1 + (real)ur * ur + (real)ui * ui);    // of u as rounded
-        if (sp.p < small || scale * f < least) {
+        if (!(sp.p > 0 && scale * f >= (fp32 ? BF_LEAST32 : BF_LEAST64))) {
+            // with the scale so far in the matrix, the pass begins anew at 1 (times what p and b
+            // lost in their rounding)
+            const cplx b = sp.b * scale;
+            const double pr = round_to((double)(sp.p * scale)), br = round_to((double)b.real()),
+                         bi = round_to((double)b.imag());
             o.kind = BF_SROT;
-            o.coef = coef({(double)sp.p});
-            set_u(o, (double)sp.b.real(), (double)sp.b.imag());
+            o.coef = coef({pr});
+            set_u(o, br, bi);
+            scale *= std::sqrt((sp.p * sp.p + std::norm(sp.b)) / ((real)pr * pr + (real)br * br + (real)bi * bi));
         } else {
             scale *= f * sp.norm;
             set_u(o, ur, ui);

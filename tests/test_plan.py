@@ -546,3 +546,25 @@ def test_butterfly_plan_of_a_circuit_with_many_cuts(emu):
     period = stats[200] - stats[100]
     assert stats[31000][0] > 32767
     assert np.array_equal((stats[31000] - stats[100])[:4] * 100, period[:4] * 30900), stats
+
+
+@pytest.mark.parametrize("precision,factor", [(1, 1.0), (1, 1e16), (1, 1e20), (1, 2e35), (0, 1e16), (0, 1e240), (0, 1e290)])
+def test_butterfly_plan_keeps_large_amplitudes_finite(emu, oracle, precision, factor):
+    """Gates with p = cos(theta / 2) = 0.02, which grow what is left unscaled most, between
+    phases, on amplitudes up to `factor`: the same state to rounding, up to the range that
+    bfly.h states."""
+    n = 13
+    gl = []
+    for q in list(range(n)) * 2:
+        gl += [G.U3(3.1, 0.2 * q, 0.1, q), G.CZ(q, (q + 1) % n), G.CZ(q, (q + 3) % n)]
+    g = G.to_array(gl)
+    st = np.random.default_rng(3).standard_normal((2, 1 << n))
+    st /= np.sqrt(np.max(st[0] ** 2 + st[1] ** 2))
+    re, im = st[0] * factor, st[1] * factor
+    stats = (ctypes.c_uint64 * 8)()
+    rc = emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), precision, 1, 1,
+                          re.ctypes.data_as(_dp), im.ctypes.data_as(_dp), stats)
+    want = oracle.run(n, g, state=(st[0], st[1]))
+    err = np.sqrt(np.sum((re / factor - want[0]) ** 2 + (im / factor - want[1]) ** 2))
+    norm = np.sqrt(np.sum(st ** 2))
+    assert rc == 0 and err <= 8 * (2.2e-16 if precision == 0 else 1.2e-7) * np.sqrt(len(g) + 26) * norm
