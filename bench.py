@@ -3,12 +3,12 @@
 
 Workload (one "step"): the n=30, depth-40 random circuit — per layer U3 with U[0,2pi)
 angles on all 30 qubits, then 15 CX on a seeded random perfect matching (1,800 gates) —
-applied in FP64 to a 16 GiB state resident in HBM, through the pair engine (two-qubit
-blocks on the FP64 tensor cores).  The state (16 GiB) is far larger than the 126 MB L2, so
+applied in FP64 to a 16 GiB state resident in HBM, through the default engine (butterflies
+in registers; --engine pairs: two-qubit blocks on the FP64 tensor cores).  The state (16 GiB) is far larger than the 126 MB L2, so
 no L2 flush is needed between steps.
 
 Printed (rank 0, one JSON line): gates/s over all ranks, the roofline of the dominant
-kernel (`k_pairs`: HBM bytes per launch and its FP64 tensor-pipe rate beside them), the
+kernel (HBM bytes per launch; with --engine pairs its FP64 tensor-pipe rate beside them), the
 reference CPU path timed on this box's
 host cores, an end-to-end figure through the C ABI with host buffers, the SM clocks seen
 during the timed region, and secondary forms (per-gate FP64 sweeps, adjoint gradients).
@@ -55,7 +55,7 @@ def parse():
     ap.add_argument("--qubits", type=int, default=N_QUBITS,
                     help="state size (smaller cases are for profiling only)")
     ap.add_argument("--tile-bits", type=int, default=12)
-    ap.add_argument("--engine", choices=["staged", "pairs"], default="pairs",
+    ap.add_argument("--engine", choices=["auto", "pairs", "staged"], default="auto",
                     help="FP64 engine of the headline step")
     ap.add_argument("--form", choices=["headline", "pergate", "fused", "qaoa", "capacity", "adjoint", "density",
                                        "config1", "tuning", "batch", "refgpu"],
@@ -311,10 +311,8 @@ def run_ours(args):
     n_gates = len(circuit)
 
     h = nat.Handle(nq, device, nat.SVB_FP64)
-    if args.engine == "pairs":
-        h.set_engine(nat.ENGINE_PAIRS, 0, 0)
-    else:
-        h.set_engine(nat.ENGINE_STAGED, args.tile_bits, 0)
+    h.set_engine({"auto": nat.ENGINE_AUTO, "pairs": nat.ENGINE_PAIRS, "staged": nat.ENGINE_STAGED}[args.engine],
+                 args.tile_bits if args.engine == "staged" else 0, 0)
     h.set_circuit(circuit)
     info = h.plan_info()
     stream = torch.cuda.current_stream(device)
@@ -355,10 +353,10 @@ def run_ours(args):
     achieved = per_launch_bytes / launch_s / 1e9
     peak, peak_kind = peaks()
     traffic = None
-    # without tensor-core blocks the pair engine runs its butterfly form
-    butterflies = args.engine == "pairs" and int(info.n_blocks) == 0
-    tfile = os.path.join(ROOT, "profiles", "pairs_fp64_traffic.txt" if args.engine == "pairs"
-                         else "staged_fp64_traffic.txt")
+    # AUTO's choice without tensor-core blocks: butterflies
+    pairs = args.engine != "staged"
+    butterflies = pairs and int(info.n_blocks) == 0
+    tfile = os.path.join(ROOT, "profiles", "pairs_fp64_traffic.txt" if pairs else "staged_fp64_traffic.txt")
     if os.path.exists(tfile) and not butterflies:
         for ln in open(tfile):
             if ln.startswith("bytes_per_launch_n30"):
@@ -366,12 +364,12 @@ def run_ours(args):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
                 "kernel": ("k_bfly (FP64 gates as butterflies in registers)" if butterflies
-                           else "k_pairs (FP64 mma.sync two-qubit blocks)" if args.engine == "pairs"
+                           else "k_pairs (FP64 mma.sync two-qubit blocks)" if pairs
                            else "k_staged<double,12>") + f" (one read+write of the {16 << nq >> 30} GiB state per launch)",
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "per_launch_bytes": per_launch_bytes, "launches_per_step": passes,
                 "gate_model_gbs": info.model_bytes / (ms_per_step / 1e3) / 1e9}
-    if args.engine == "pairs" and int(info.n_blocks) > 0:
+    if pairs and int(info.n_blocks) > 0:
         # the pair kernel is bound by the FP64 tensor cores, not by HBM: each two-qubit
         # block is 16 multiply-adds per amplitude; the rate they allow is measured live
         flops = int(info.n_blocks) * float(1 << nq) * 16 * 2
@@ -501,7 +499,7 @@ def capacity_form(device, shots=4096):
     from svsim_b200 import circuits, _native as nat
     out = {}
     uni = np.random.default_rng(1).random(shots)
-    for n, prec, eng, k, name in ((33, nat.SVB_FP64, nat.ENGINE_PAIRS, 0, "n33_fp64_pairs"),
+    for n, prec, eng, k, name in ((33, nat.SVB_FP64, nat.ENGINE_AUTO, 0, "n33_fp64"),
                                   (34, nat.SVB_FP32, nat.ENGINE_FUSED, 5, "n34_fp32_fused")):
         circ = circuits.random_matching_circuit(n, 20, seed=SEED)
         h = nat.Handle(n, device, prec)
@@ -747,7 +745,7 @@ def tuning_form(device):
     import torch
     from svsim_b200 import circuits, _native as nat
     g = circuits.random_matching_circuit(N_QUBITS, DEPTH, seed=SEED)
-    names = {0: "auto", 1: "per_gate", 2: "staged", 3: "fused", 4: "pairs"}
+    names = {0: "auto", 1: "per_gate", 2: "staged", 3: "fused", 4: "pairs", 5: "butterfly"}
     out = {}
     for prec, key in ((nat.SVB_FP64, "fp64"), (nat.SVB_FP32, "fp32")):
         h = nat.Handle(N_QUBITS, device, prec)

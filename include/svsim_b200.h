@@ -43,14 +43,18 @@ typedef enum svb_precision {
 } svb_precision;
 
 typedef enum svb_engine {
-    SVB_ENGINE_AUTO = 0,      /* n >= 12 without SRN: pairs (FP64) or fused (FP32); else
-                                 staged for n >= 10 (FP32: 11), per-gate below */
+    SVB_ENGINE_AUTO = 0,      /* n >= 12 without SRN: pairs (FP64) or fused (FP32), or
+                                 butterflies where those are faster; else staged for
+                                 n >= 10 (FP32: 11), per-gate below */
     SVB_ENGINE_PER_GATE = 1,  /* one HBM sweep per elementary gate, as the reference */
     SVB_ENGINE_STAGED = 2,    /* many gates per HBM sweep through a shared-memory tile */
-    SVB_ENGINE_FUSED = 3,     /* gates fused into dense k-qubit blocks (FP32 only); circuits of
-                                 mostly phases run as butterflies when no width is asked for */
-    SVB_ENGINE_PAIRS = 4      /* FP64 two-qubit blocks on the FP64 tensor cores, or butterflies
-                                 in registers where those are faster (FP64, n >= 12, no SRN) */
+    SVB_ENGINE_FUSED = 3,     /* gates fused into dense k-qubit blocks (FP32 only) */
+    SVB_ENGINE_PAIRS = 4,     /* FP64 two-qubit blocks on the FP64 tensor cores (FP64, n >= 12,
+                                 no SRN) */
+    SVB_ENGINE_BUTTERFLY = 5  /* gates split at CXs, in registers (n >= 12 FP64, 13 FP32; no SRN,
+                                 R or two-qubit matrices).  Amplitudes up to 1e290 (FP64) and
+                                 3e35 (FP32) stay finite.  Unlike the fused engine's blocks it
+                                 leaves the state's norm as it is */
 } svb_engine;
 
 /* One gate: the fields of the reference's class Gate (svsim_nvgpu_sin.cuh:99-188)
@@ -89,11 +93,11 @@ typedef struct svb_plan_info {
     double   model_bytes;      /* per-gate-model algorithmic bytes of one run */
     double   moved_bytes;      /* bytes the plan reads+writes in HBM per run */
     uint64_t plan_bytes;       /* bytes of plan descriptors uploaded by svb_set_circuit */
-    int      engine;           /* engine the plan was built for */
+    int      engine;           /* engine the plan was built for (butterflies: PAIRS for FP64
+                                  states, FUSED for FP32, with n_blocks 0) */
     int      tile_bits;        /* local qubits per tile */
     uint64_t n_blocks;         /* tensor-core blocks per run: two-qubit blocks of the pair
-                                  engine, fused blocks of the fused engine; 0 otherwise, and
-                                  where either runs its butterfly form */
+                                  engine, fused blocks of the fused engine; 0 otherwise */
 } svb_plan_info;
 
 typedef struct svb_sim svb_sim;
@@ -141,8 +145,8 @@ typedef struct svb_tune_result {
 /* Autotuner (no reference counterpart; the reference fixes its launch shape,
  * svsim_nvgpu_sin.cuh:309-316, config.hpp:48): times every engine configuration that can
  * run the circuit on this handle (per-gate for n <= 26; staged at each tile size; the pair
- * engine for FP64 or the fused engine at k = 3..6 for FP32, when the circuit has no SRN)
- * on its first min(n_gates, 360) gates, one warm-up and one timed run each, and keeps the
+ * engine for FP64 or the fused engine at k = 3..6 for FP32, when the circuit has no SRN,
+ * and butterflies where they can) on its first min(n_gates, 360) gates, one warm-up and one timed run each, and keeps the
  * fastest for this circuit structure (qubit count, precision, and the ops and qubits of
  * every elementary op; angles ignored): from then on svb_set_circuit with
  * SVB_ENGINE_AUTO picks it for any circuit of that structure on this device.  The handle

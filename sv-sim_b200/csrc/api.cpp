@@ -470,7 +470,7 @@ svb_status svb_reset_state(svb_sim* s)
 svb_status svb_set_engine(svb_sim* s, int engine, int tile_bits, int fusion_width)
 {
     if (!s) return invalid("svb_set_engine: NULL handle");
-    if (engine < SVB_ENGINE_AUTO || engine > SVB_ENGINE_PAIRS)
+    if (engine < SVB_ENGINE_AUTO || engine > SVB_ENGINE_BUTTERFLY)
         return invalid("svb_set_engine: unknown engine");
     if (engine == SVB_ENGINE_FUSED && s->precision != SVB_FP32)
         return invalid("svb_set_engine: the fused engine runs FP32 states");
@@ -545,7 +545,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         if (it != g_tuned.end()) {
             engine = it->second.engine;
             if (it->second.tile_bits) M = it->second.tile_bits;
-            if (engine == SVB_ENGINE_FUSED) fusion = it->second.fusion_width;
+            if (it->second.fusion_width) fusion = it->second.fusion_width;
         }
     }
     if (has_m4) {
@@ -557,13 +557,25 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             return SVB_ERR_UNSUPPORTED;
         }
     }
+    bool bfly = engine == SVB_ENGINE_BUTTERFLY;
+    if (bfly) {
+        if (!bfly_supported(s->eops, n, s->precision)) {
+            set_error("svb_set_circuit: butterflies need >= 12 qubits (13 in FP32) and no SRN or R");
+            return SVB_ERR_UNSUPPORTED;
+        }
+        engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
+    }
     if (engine == SVB_ENGINE_AUTO) {
         // Circuits of >= 12 qubits without SRN (which has no matrix) go to the tensor cores:
         // FP64 to the pair engine, FP32 to the fused engine (2x the staged engine at n = 24
-        // and 30); otherwise the staged engine, per-gate below its tile
-        if (n >= PR_TILE_BITS && fusable(s->eops))
+        // and 30), or to butterflies where those are faster (FP32: unless a fusion width is
+        // asked for); otherwise the staged engine, per-gate below its tile
+        if (n >= PR_TILE_BITS && fusable(s->eops)) {
             engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
-        else engine = (staged_supported(s->precision, M) && n >= M) ? SVB_ENGINE_STAGED : SVB_ENGINE_PER_GATE;
+            bfly = (engine == SVB_ENGINE_PAIRS || fusion == 0) && bfly_preferred(s->eops, n, s->precision);
+        } else {
+            engine = (staged_supported(s->precision, M) && n >= M) ? SVB_ENGINE_STAGED : SVB_ENGINE_PER_GATE;
+        }
     }
     if (engine == SVB_ENGINE_FUSED) {
         if (s->precision != SVB_FP32 || n < FT_TILE_BITS) {
@@ -598,11 +610,15 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     s->info.state_bytes = sb;
     s->info.model_bytes = 2.0 * sb * sweeps;
     s->info.engine = engine;
-    // the butterfly form of the pair engine (FP64) and, where no fusion width is asked for, of
-    // the fused engine (FP32), for the circuits it is faster on
     BfPlan B;
-    if ((engine == SVB_ENGINE_PAIRS || (engine == SVB_ENGINE_FUSED && fusion == 0)) &&
-        bfly_preferred(s->eops, n, s->precision) && plan_bfly(s->eops, n, s->precision, B, true)) {
+    if (bfly && !plan_bfly(s->eops, n, s->precision, B, true)) {
+        if (s->engine_req == SVB_ENGINE_BUTTERFLY) {
+            set_error("svb_set_circuit: the butterfly planner rejected the circuit");
+            return SVB_ERR_UNSUPPORTED;
+        }
+        bfly = false;
+    }
+    if (bfly) {
         // an earlier circuit's kernels may still read the buffer, on any stream
         SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
         SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly), "plan upload");
@@ -1001,10 +1017,9 @@ extern "C" svb_status svb_autotune(svb_sim* s, const svb_gate* gates, size_t n_g
         if (n >= M) cands.push_back({SVB_ENGINE_STAGED, M, 0});
     if (n >= PR_TILE_BITS && matrices) {
         if (fp64) cands.push_back({SVB_ENGINE_PAIRS, 0, 0});
-        else {
-            if (bfly_preferred(eops, n, s->precision)) cands.push_back({SVB_ENGINE_FUSED, 0, 0});
+        else
             for (int k = FT_MIN_K; k <= FT_MAX_K; k++) cands.push_back({SVB_ENGINE_FUSED, 0, k});
-        }
+        if (bfly_supported(eops, n, s->precision)) cands.push_back({SVB_ENGINE_BUTTERFLY, 0, 0});
     }
     // the prefix timed: the whole circuit up to 360 gates (the choice holds for the structure)
     const size_t P = std::min<size_t>(n_gates, 360);

@@ -115,3 +115,51 @@ def test_packed_control_onto_a_shared_register(oracle, n, t, y):
     re, im = h.get_state()
     want = oracle.run(n, g, state=(st[0], st[1]))
     assert np.sqrt(np.sum((re - want[0]) ** 2 + (im - want[1]) ** 2)) <= 1.2e-7
+
+
+def test_either_form_can_be_named(oracle):
+    """The tensor-core engines by name run blocks where the default runs butterflies, and
+    butterflies by name run where the default runs blocks; both give the same state."""
+    from svsim_b200 import _native as nat
+    from svsim_b200._native import SvbError
+    random_circuit = circuits.random_matching_circuit(16, 4, seed=1)
+    for prec, blocks, tol in ((nat.SVB_FP64, nat.ENGINE_PAIRS, 1e-13), (nat.SVB_FP32, nat.ENGINE_FUSED, 2e-6)):
+        for g in (qft(16, 1), random_circuit):
+            want = oracle.run(16, g)
+            for engine in (nat.ENGINE_AUTO, blocks, nat.ENGINE_BUTTERFLY):
+                h = nat.Handle(16, 0, prec)
+                h.set_engine(engine)
+                h.set_circuit(g)
+                butterflies = engine == nat.ENGINE_BUTTERFLY or (engine == nat.ENGINE_AUTO and g is not random_circuit)
+                assert (h.plan_info().n_blocks == 0) == butterflies and h.plan_info().engine == blocks
+                h.run()
+                re, im = h.get_state()
+                assert np.max(np.abs(re - want[0])) < tol and np.max(np.abs(im - want[1])) < tol
+    big = nat.Handle(25, 0, nat.SVB_FP64)
+    big.set_engine(nat.ENGINE_PAIRS)
+    big.set_circuit(circuits.random_matching_circuit(25, 2, seed=1))
+    assert big.plan_info().n_blocks > 0
+    for n, prec, gl in ((11, nat.SVB_FP64, [G.H(0)]), (12, nat.SVB_FP32, [G.H(0)]), (14, nat.SVB_FP64, [G.SRN(0)]),
+                        (14, nat.SVB_FP64, [G.R(0.5, 0)])):
+        h = nat.Handle(n, 0, prec)
+        h.set_engine(nat.ENGINE_BUTTERFLY)
+        with pytest.raises(SvbError):
+            h.set_circuit(G.to_array(gl))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_autotune_times_both_forms(precision):
+    """The autotuner has both forms among its candidates, and its choice is a name that
+    set_engine takes and that gives the plan AUTO then has."""
+    from svsim_b200 import _native as nat
+    n = 17                               # a structure that no other test leaves to AUTO
+    g = qft(n, 1)
+    h = nat.Handle(n, 0, precision)
+    r = h.autotune(g)
+    # per gate, three tile sizes, and the pair engine or the fused engine at four widths, and butterflies
+    assert r.candidates == (6 if precision == 0 else 9)
+    tuned = h.plan_info().n_blocks
+    f = nat.Handle(n, 0, precision)
+    f.set_engine(r.engine, r.tile_bits, r.fusion_width)
+    f.set_circuit(g)
+    assert f.plan_info().n_blocks == tuned and f.plan_info().engine == h.plan_info().engine

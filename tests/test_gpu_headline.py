@@ -151,6 +151,21 @@ def test_headline_fp64_matches_reference(golden, engine):
         h.close()
 
 
+def test_headline_default_matches_reference(golden):
+    """The default engine's state (butterflies): the same bounds."""
+    nat = native()
+    h = run_headline(golden, nat.ENGINE_AUTO)
+    try:
+        assert h.plan_info().n_blocks == 0
+        max_abs, err2, cs, dnorm = compare_with_golden(h, golden)
+        print(f"butterflies: max|d amp| {max_abs:.3e}, ||e||^2 (sketch) {err2:.3e}, checksum {cs:.3e}, norm {dnorm:.3e}")
+        assert max_abs <= FP64_TOL and err2 <= FP64_TOL and cs <= 1e-10 and dnorm <= FP64_TOL
+        bad, near = sample_mismatches(h, golden)
+        assert bad == near and bad <= 40, (bad, near)
+    finally:
+        h.close()
+
+
 @pytest.mark.parametrize("k", [4, 5, 6])
 def test_headline_fused_fp32_matches_reference(golden, k):
     nat = native()
