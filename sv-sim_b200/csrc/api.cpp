@@ -450,7 +450,7 @@ svb_status svb_destroy(svb_sim* s)
     free_scratch(s);
     cudaFree(s->state);
     cudaFree(s->d_small);
-    if (s->capture_stream) cudaStreamDestroy(s->capture_stream);
+    if (s->own_stream) cudaStreamDestroy(s->own_stream);
     delete s;
     return SVB_OK;
 }
@@ -522,9 +522,37 @@ std::array<uint64_t, 4> structure_key(const Sim* s, const std::vector<EOp>& eops
     return {(uint64_t)s->device, (uint64_t)s->n | ((uint64_t)s->precision << 32), (uint64_t)eops.size(), h};
 }
 
+svb_status own_stream(Sim* s)
+{
+    if (!s->own_stream)
+        SVB_CUDA(cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    return SVB_OK;
+}
+
+// A new device buffer of a plan with the host's values in it, of at least `least` of them.
+// The copy is on the handle's own stream, behind no other handle's work; set_circuit_lowered
+// ends with a wait for that stream, since a copy from pageable memory can return before it
+// has reached the device and the circuit may run on any stream.
+template <typename T>
+svb_status upload(Sim* s, T** dst, const std::vector<T>& v, size_t least = 1)
+{
+    SVB_CUDA(cudaMalloc(dst, std::max(least, v.size()) * sizeof(T)), "cudaMalloc(plan)");
+    if (!v.empty())
+        SVB_CUDA(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s->own_stream),
+                 "plan upload");
+    return SVB_OK;
+}
+
+#define SVB_TRY(call)                                   \
+    do {                                                \
+        const svb_status r_ = (call);                   \
+        if (r_ != SVB_OK) return r_;                    \
+    } while (0)
+
 svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* gates, size_t n_gates, double sweeps)
 {
     SVB_CUDA(cudaSetDevice(s->device), "cudaSetDevice");
+    SVB_TRY(own_stream(s));
     bool has_m4 = false;
     for (const EOp& e : eops) has_m4 |= e.form == F_M4;
     std::vector<Mat4> mats;
@@ -621,7 +649,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     if (bfly) {
         // an earlier circuit's kernels may still read the buffer, on any stream
         SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
-        SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly), "plan upload");
+        SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly, s->own_stream), "plan upload");
         s->bfly = true;
         s->info.n_passes = B.passes.size();
         s->info.tile_bits = B.tile_bits;
@@ -635,29 +663,13 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         if (k == F6_K) plan_fused6(s->eops, n, s->fused);
         else plan_fused(s->eops, n, k, s->fused);
         const FusedPlan& F = s->fused;
-        SVB_CUDA(cudaMalloc(&s->dfused.passes, std::max<size_t>(1, F.passes.size()) * sizeof(FusedPass)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dfused.blocks, std::max<size_t>(1, F.blocks.size()) * sizeof(FusedBlock)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dfused.gates, std::max<size_t>(4, F.gates.size()) * sizeof(float)),
-                 "cudaMalloc(plan)");
+        SVB_TRY(upload(s, &s->dfused.passes, F.passes));
+        SVB_TRY(upload(s, &s->dfused.blocks, F.blocks));
+        SVB_TRY(upload(s, &s->dfused.gates, F.gates, 4));
+        if (!F.passes6.empty()) SVB_TRY(upload(s, &s->dfused.passes6, F.passes6));
         SVB_CUDA(cudaMalloc(&s->dfused.err, sizeof(int)), "cudaMalloc(flag)");
-        SVB_CUDA(cudaMemset(s->dfused.err, 0, sizeof(int)), "cudaMemset");
+        SVB_CUDA(cudaMemsetAsync(s->dfused.err, 0, sizeof(int), s->own_stream), "cudaMemset");
         SVB_CUDA(cudaMalloc(&s->dfused.norm_partial, REDUCE_BLOCKS * sizeof(double)), "cudaMalloc(norm)");
-        if (!F.passes.empty())
-            SVB_CUDA(cudaMemcpy(s->dfused.passes, F.passes.data(), F.passes.size() * sizeof(FusedPass),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!F.blocks.empty())
-            SVB_CUDA(cudaMemcpy(s->dfused.blocks, F.blocks.data(), F.blocks.size() * sizeof(FusedBlock),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!F.gates.empty())
-            SVB_CUDA(cudaMemcpy(s->dfused.gates, F.gates.data(), F.gates.size() * sizeof(float),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!F.passes6.empty()) {
-            SVB_CUDA(cudaMalloc(&s->dfused.passes6, F.passes6.size() * sizeof(Fused6Pass)), "cudaMalloc(plan)");
-            SVB_CUDA(cudaMemcpy(s->dfused.passes6, F.passes6.data(), F.passes6.size() * sizeof(Fused6Pass),
-                                cudaMemcpyHostToDevice), "plan upload");
-        }
         const size_t np = F.n_passes();
         s->info.n_passes = np;
         s->info.tile_bits = k == F6_K ? F6_TILE_BITS : FT_TILE_BITS;
@@ -672,25 +684,10 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             return SVB_ERR_UNSUPPORTED;
         }
         const PairPlan& R = s->pairs;
-        SVB_CUDA(cudaMalloc(&s->dpairs.passes, std::max<size_t>(1, R.passes.size()) * sizeof(PairPass)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dpairs.ops, std::max<size_t>(1, R.ops.size()) * sizeof(PairOp)), "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dpairs.layouts, std::max<size_t>(1, R.layouts.size()) * sizeof(DevStage)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dpairs.gates, std::max<size_t>(2, R.gates.size()) * sizeof(double)),
-                 "cudaMalloc(plan)");
-        if (!R.passes.empty())
-            SVB_CUDA(cudaMemcpy(s->dpairs.passes, R.passes.data(), R.passes.size() * sizeof(PairPass),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!R.ops.empty())
-            SVB_CUDA(cudaMemcpy(s->dpairs.ops, R.ops.data(), R.ops.size() * sizeof(PairOp), cudaMemcpyHostToDevice),
-                     "plan upload");
-        if (!R.layouts.empty())
-            SVB_CUDA(cudaMemcpy(s->dpairs.layouts, R.layouts.data(), R.layouts.size() * sizeof(DevStage),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!R.gates.empty())
-            SVB_CUDA(cudaMemcpy(s->dpairs.gates, R.gates.data(), R.gates.size() * sizeof(double),
-                                cudaMemcpyHostToDevice), "plan upload");
+        SVB_TRY(upload(s, &s->dpairs.passes, R.passes));
+        SVB_TRY(upload(s, &s->dpairs.ops, R.ops));
+        SVB_TRY(upload(s, &s->dpairs.layouts, R.layouts));
+        SVB_TRY(upload(s, &s->dpairs.gates, R.gates, 2));
         s->dpairs.stage_bytes = R.stage_bytes;
         s->info.n_passes = R.passes.size();
         s->info.tile_bits = PR_TILE_BITS;
@@ -702,21 +699,9 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         const int G = s->precision == SVB_FP64 ? 3 : 4;
         plan_staged(s->eops, n, M, G, s->staged);
         const StagedPlan& P = s->staged;
-        SVB_CUDA(cudaMalloc(&s->dplan.passes, std::max<size_t>(1, P.passes.size()) * sizeof(DevPass)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dplan.stages, std::max<size_t>(1, P.stages.size()) * sizeof(DevStage)),
-                 "cudaMalloc(plan)");
-        SVB_CUDA(cudaMalloc(&s->dplan.ops, std::max<size_t>(1, P.ops.size()) * sizeof(DevOp)),
-                 "cudaMalloc(plan)");
-        if (!P.passes.empty())
-            SVB_CUDA(cudaMemcpy(s->dplan.passes, P.passes.data(), P.passes.size() * sizeof(DevPass),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!P.stages.empty())
-            SVB_CUDA(cudaMemcpy(s->dplan.stages, P.stages.data(), P.stages.size() * sizeof(DevStage),
-                                cudaMemcpyHostToDevice), "plan upload");
-        if (!P.ops.empty())
-            SVB_CUDA(cudaMemcpy(s->dplan.ops, P.ops.data(), P.ops.size() * sizeof(DevOp),
-                                cudaMemcpyHostToDevice), "plan upload");
+        SVB_TRY(upload(s, &s->dplan.passes, P.passes));
+        SVB_TRY(upload(s, &s->dplan.stages, P.stages));
+        SVB_TRY(upload(s, &s->dplan.ops, P.ops));
         s->info.n_passes = P.passes.size();
         s->info.tile_bits = M;
         s->info.plan_bytes = P.passes.size() * sizeof(DevPass) + P.stages.size() * sizeof(DevStage) +
@@ -749,7 +734,8 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             // an earlier circuit's kernel may still read the buffer, on any stream
             SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
             SVB_CUDA(grow(s->plan_buf, host.size()), "cudaMalloc(plan)");
-            SVB_CUDA(cudaMemcpy(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice), "plan upload");
+            SVB_CUDA(cudaMemcpyAsync(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice, s->own_stream),
+                     "plan upload");
             s->small_ops = static_cast<const SmallOp*>(s->plan_buf.p);
             s->small_mats = reinterpret_cast<const double*>(static_cast<unsigned char*>(s->plan_buf.p) + ob);
             s->info.n_passes = 1;
@@ -757,6 +743,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             s->info.moved_bytes = 2.0 * sb;
         }
     }
+    SVB_CUDA(cudaStreamSynchronize(s->own_stream), "plan upload");
     s->have_circuit = true;
     return SVB_OK;
 }
@@ -792,14 +779,11 @@ svb_status svb_run(svb_sim* s, void* stream)
     if (s->info.n_passes == 0) return SVB_OK;
     if (use_graph(s)) {
         if (!s->graph) {
-            if (!s->capture_stream)
-                SVB_CUDA(cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking),
-                         "cudaStreamCreate");
-            SVB_CUDA(cudaStreamBeginCapture(s->capture_stream, cudaStreamCaptureModeThreadLocal),
+            SVB_CUDA(cudaStreamBeginCapture(s->own_stream, cudaStreamCaptureModeThreadLocal),
                      "cudaStreamBeginCapture");
-            svb_status rc = launch_all(s, s->capture_stream);
+            svb_status rc = launch_all(s, s->own_stream);
             cudaGraph_t g = nullptr;
-            cudaError_t e = cudaStreamEndCapture(s->capture_stream, &g);
+            cudaError_t e = cudaStreamEndCapture(s->own_stream, &g);
             if (rc != SVB_OK) { if (g) cudaGraphDestroy(g); return rc; }
             if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
             e = cudaGraphInstantiate(&s->graph, g, 0);

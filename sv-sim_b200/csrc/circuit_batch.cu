@@ -793,6 +793,8 @@ svb_status cb_create_with(svb_circuit_batch* proto, int MB, int threads, bool us
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_pgates, std::max<size_t>(1, PP.gates.size()) * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_energy, std::max<size_t>(1, b->n_circ) * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_err, 4 * sizeof(unsigned));
+    // the batch runs on a stream of its own, and copies from pageable memory can return early
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) return fail("allocation", e);
     if (!b->plan.ops.empty()) std::memcpy(b->h_ops, b->plan.ops.data(), b->plan.ops.size() * sizeof(CbOp));
     if (!PP.gates.empty()) std::memcpy(b->h_pgates, PP.gates.data(), PP.gates.size() * sizeof(double));

@@ -535,14 +535,14 @@ struct Sim {
     PairPlan pairs;
     DevPairBuffers dpairs;
     bool bfly = false;             // the pair or fused engine's plan is a butterfly plan
-    DevBfBuffers dbfly;            // into bfly_buf
+    DevBfBuffers dbfly;            // into plan_buf
     GrowBuf plan_buf;              // the butterfly plan's or the small state's ops, kept from
                                    // circuit to circuit
     const SmallOp* small_ops = nullptr;   // per-gate engine on a small state: into plan_buf
     const double* small_mats = nullptr;
     bool have_circuit = false;
     cudaGraphExec_t graph = nullptr;
-    cudaStream_t capture_stream = nullptr;
+    cudaStream_t own_stream = nullptr;    // uploads of plans and capture of their graphs
     svb_plan_info info{};
     // scratch
     MeasureScratch mscr;

@@ -163,3 +163,26 @@ def test_autotune_times_both_forms(precision):
     f.set_engine(r.engine, r.tile_bits, r.fusion_width)
     f.set_circuit(g)
     assert f.plan_info().n_blocks == tuned and f.plan_info().engine == h.plan_info().engine
+
+
+@pytest.mark.parametrize("engine,precision,n", [("BUTTERFLY", 0, 15), ("BUTTERFLY", 1, 15), ("PAIRS", 0, 14), ("FUSED", 1, 14),
+                                                ("STAGED", 0, 14), ("PER_GATE", 0, 8)])
+def test_a_run_on_a_side_stream_straight_after_the_upload(oracle, engine, precision, n):
+    """set_circuit returns with the plan on the device: a run on a stream that does not wait for
+    the default one, with circuits of different length in turn (a reused plan buffer would hold
+    the earlier one's)."""
+    import torch
+    from svsim_b200 import _native as nat
+    stream = torch.cuda.Stream()
+    h = nat.Handle(n, 0, precision)
+    h.set_engine(getattr(nat, "ENGINE_" + engine))
+    want = None
+    for i in range(12):
+        g = circuits.random_matching_circuit(n, 2 + 5 * (i % 3), seed=i)
+        want = oracle.run(n, g, state=want)
+        h.set_circuit(g)
+        h.run(stream.cuda_stream)
+    stream.synchronize()
+    re, im = h.get_state()
+    tol = 1e-5 if precision else 1e-12
+    assert np.max(np.abs(re - want[0])) < tol and np.max(np.abs(im - want[1])) < tol
