@@ -451,6 +451,7 @@ svb_status svb_destroy(svb_sim* s)
     cudaFree(s->state);
     cudaFree(s->d_small);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
+    if (s->plan_read) cudaEventDestroy(s->plan_read);
     delete s;
     return SVB_OK;
 }
@@ -540,6 +541,33 @@ svb_status upload(Sim* s, T** dst, const std::vector<T>& v, size_t least = 1)
     if (!v.empty())
         SVB_CUDA(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s->own_stream),
                  "plan upload");
+    return SVB_OK;
+}
+
+// Runs of a handle change one state, so the program orders them: the last one's end is the
+// end of all.  A run captured into a caller's graph has no such end.
+svb_status mark_plan_buf(Sim* s, cudaStream_t st)
+{
+    if (!s->plan_read)
+        SVB_CUDA(cudaEventCreateWithFlags(&s->plan_read, cudaEventDisableTiming), "cudaEventCreate");
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        s->plan_reader = Sim::CAPTURED;
+    } else if (s->plan_reader != Sim::CAPTURED) {
+        SVB_CUDA(cudaEventRecord(s->plan_read, st), "cudaEventRecord");
+        s->plan_reader = Sim::READ;
+    }
+    return SVB_OK;
+}
+
+// Before plan_buf is written again: waits for the runs that read it, and for no other
+// handle's work.
+svb_status wait_plan_buf(Sim* s)
+{
+    if (s->plan_reader == Sim::READ) SVB_CUDA(cudaEventSynchronize(s->plan_read), "kernel execution");
+    else if (s->plan_reader == Sim::CAPTURED) SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+    s->plan_reader = Sim::UNREAD;
     return SVB_OK;
 }
 
@@ -647,8 +675,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         bfly = false;
     }
     if (bfly) {
-        // an earlier circuit's kernels may still read the buffer, on any stream
-        SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+        SVB_TRY(wait_plan_buf(s));
         SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly, s->own_stream), "plan upload");
         s->bfly = true;
         s->info.n_passes = B.passes.size();
@@ -731,8 +758,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
                 so[i].mat = e.mat;
             }
             if (mb) std::memcpy(host.data() + ob, s->mats.data(), mb);
-            // an earlier circuit's kernel may still read the buffer, on any stream
-            SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+            SVB_TRY(wait_plan_buf(s));
             SVB_CUDA(grow(s->plan_buf, host.size()), "cudaMalloc(plan)");
             SVB_CUDA(cudaMemcpyAsync(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice, s->own_stream),
                      "plan upload");
@@ -791,9 +817,11 @@ svb_status svb_run(svb_sim* s, void* stream)
             if (e != cudaSuccess) { s->graph = nullptr; return cuda_fail(e, "cudaGraphInstantiate"); }
         }
         SVB_CUDA(cudaGraphLaunch(s->graph, st), "cudaGraphLaunch");
-        return SVB_OK;
+    } else {
+        const svb_status rc = launch_all(s, st);
+        if (rc != SVB_OK) return rc;
     }
-    return launch_all(s, st);
+    return s->bfly || s->small_ops ? mark_plan_buf(s, st) : SVB_OK;
 }
 
 svb_status svb_synchronize(svb_sim* s)

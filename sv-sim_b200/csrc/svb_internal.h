@@ -538,6 +538,8 @@ struct Sim {
     DevBfBuffers dbfly;            // into plan_buf
     GrowBuf plan_buf;              // the butterfly plan's or the small state's ops, kept from
                                    // circuit to circuit
+    enum { UNREAD, READ, CAPTURED } plan_reader = UNREAD;    // runs that read plan_buf
+    cudaEvent_t plan_read = nullptr;      // READ: behind the last of them
     const SmallOp* small_ops = nullptr;   // per-gate engine on a small state: into plan_buf
     const double* small_mats = nullptr;
     bool have_circuit = false;

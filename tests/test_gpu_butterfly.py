@@ -186,3 +186,31 @@ def test_a_run_on_a_side_stream_straight_after_the_upload(oracle, engine, precis
     re, im = h.get_state()
     tol = 1e-5 if precision else 1e-12
     assert np.max(np.abs(re - want[0])) < tol and np.max(np.abs(im - want[1])) < tol
+
+
+@pytest.mark.parametrize("engine,n", [("PER_GATE", 8), ("BUTTERFLY", 16)])
+def test_an_upload_does_not_wait_for_another_handle(engine, n):
+    """set_circuit waits for its own handle's runs where it reuses their buffer: not for another
+    handle's, here about half a second of them queued on a stream of their own."""
+    import torch
+    from svsim_b200 import _native as nat
+    busy = nat.Handle(28, 0, nat.SVB_FP64)
+    busy.set_circuit(circuits.random_matching_circuit(28, 20, seed=1))
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    h.set_engine(getattr(nat, "ENGINE_" + engine))
+    own, side = torch.cuda.Stream(), torch.cuda.Stream()
+    g = [circuits.random_matching_circuit(n, 3, seed=s) for s in range(2)]
+    for b, depth in ((busy, 3), (h, 8)):     # what the first run loads, and a buffer for all
+        b.set_circuit(circuits.random_matching_circuit(b.n, depth, seed=2))
+        b.run(own.cuda_stream)
+        b.sync()
+    for _ in range(40):
+        busy.run(side.cuda_stream)
+    done = torch.cuda.Event()
+    done.record(side)
+    for i in range(4):
+        h.set_circuit(g[i % 2])
+        h.run(own.cuda_stream)
+    h.set_circuit(g[0])
+    assert not done.query()
+    torch.cuda.synchronize()
