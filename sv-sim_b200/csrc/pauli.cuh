@@ -67,7 +67,8 @@ __device__ __forceinline__ double pauli_energy(const typename VecOf<T>::type* __
         }
     }
 #pragma unroll
-    for (int u = 0; u < PAULI_U; u++) acc += diag[u] * (ar[u] * ar[u] + ai[u] * ai[u]);
+    for (int u = 0; u < PAULI_U; u++)       // 0 without Z strings, also where |a|^2 is no double
+        acc += diag[u] * ar[u] * ar[u] + diag[u] * ai[u] * ai[u];
     return acc;
 }
 

@@ -72,3 +72,18 @@ def test_pauli_sums(oracle, n, count):
     binding["idx"] = -1
     ea, _ = h.adjoint(g, binding, 0, t)
     assert abs(ea - want) <= bound
+
+
+@pytest.mark.parametrize("n", [1, 5, 13])
+def test_pauli_sums_of_amplitudes_whose_squares_overflow(n):
+    """X and Y strings multiply two different amplitudes: 1e200 and 1e-190 give a number where
+    |1e200|^2 is none."""
+    from svsim_b200 import _native as nat
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    re, im = np.full(1 << n, 1e-190), np.full(1 << n, 2e-190)
+    re[0] = 1e200
+    h.set_state(re, im)
+    t = np.zeros(2, dtype=PAULI_DTYPE)
+    t[0], t[1] = (0.5, 1, 0), (0.25, 1, 1)
+    # <X_0> and <Y_0> of the pair (0, 1): 2 * 1e200 * 1e-190 and 2 * 1e200 * 2e-190
+    assert abs(h.expectation(t) - (0.5 * 2e10 + 0.25 * 4e10)) <= 1e-4
