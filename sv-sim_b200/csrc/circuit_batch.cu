@@ -747,10 +747,11 @@ cudaError_t cb_enqueue(svb_circuit_batch* b, cudaStream_t s)
 }
 
 template <typename Tp>
-cudaError_t upload(Tp** dst, const std::vector<Tp>& v)
+cudaError_t upload(Tp** dst, const std::vector<Tp>& v, cudaStream_t s)
 {
     cudaError_t e = cudaMalloc(dst, std::max<size_t>(1, v.size()) * sizeof(Tp));
-    if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(Tp), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !v.empty())
+        e = cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(Tp), cudaMemcpyHostToDevice, s);
     return e;
 }
 
@@ -771,30 +772,30 @@ svb_status cb_create_with(svb_circuit_batch* proto, int MB, int threads, bool us
     std::string err;
     if (!cb_build_plan(b, b->gates.data(), MB, use_pairs, b->plan, err)) return fail(err, cudaSuccess);
     const size_t amp = b->precision == SVB_FP64 ? 16 : 8;
-    cudaError_t e = cudaMalloc(&b->pool, std::max<uint64_t>(1, b->plan.pool_amps) * amp);
-    if (e == cudaSuccess) e = upload(&b->d_circ, b->plan.circ);
-    if (e == cudaSuccess) e = upload(&b->d_passes, b->plan.passes);
-    if (e == cudaSuccess) e = upload(&b->d_ops, b->plan.ops);
-    if (e == cudaSuccess) e = upload(&b->d_items, b->plan.items);
-    if (e == cudaSuccess) e = upload(&b->d_phase_off, b->plan.phase_off);
-    if (e == cudaSuccess) e = upload(&b->d_terms, b->terms);
-    if (e == cudaSuccess) e = upload(&b->d_chunk_circ, b->plan.chunk_circ);
+    // the uploads on the stream that the batch runs on: in order with its first evaluation
+    cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&b->pool, std::max<uint64_t>(1, b->plan.pool_amps) * amp);
+    if (e == cudaSuccess) e = upload(&b->d_circ, b->plan.circ, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_passes, b->plan.passes, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_ops, b->plan.ops, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_items, b->plan.items, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_phase_off, b->plan.phase_off, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_terms, b->terms, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_chunk_circ, b->plan.chunk_circ, b->stream);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_partial, std::max<size_t>(1, b->plan.chunk_circ.size()) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_energy, std::max<size_t>(1, b->n_circ) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_bar, 4 * sizeof(unsigned));
     const CbPairPlan& PP = b->plan.pairs;
-    if (e == cudaSuccess) e = upload(&b->d_ppasses, PP.passes);
-    if (e == cudaSuccess) e = upload(&b->d_pops, PP.ops);
-    if (e == cudaSuccess) e = upload(&b->d_playouts, PP.layouts);
-    if (e == cudaSuccess) e = upload(&b->d_pgates, PP.gates);
-    if (e == cudaSuccess) e = upload(&b->d_pitems, PP.items);
-    if (e == cudaSuccess) e = upload(&b->d_pphase_off, PP.phase_off);
+    if (e == cudaSuccess) e = upload(&b->d_ppasses, PP.passes, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_pops, PP.ops, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_playouts, PP.layouts, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_pgates, PP.gates, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_pitems, PP.items, b->stream);
+    if (e == cudaSuccess) e = upload(&b->d_pphase_off, PP.phase_off, b->stream);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_ops, std::max<size_t>(1, b->plan.ops.size()) * sizeof(CbOp));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_pgates, std::max<size_t>(1, PP.gates.size()) * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_energy, std::max<size_t>(1, b->n_circ) * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_err, 4 * sizeof(unsigned));
-    // the batch runs on a stream of its own, and copies from pageable memory can return early
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) return fail("allocation", e);
     if (!b->plan.ops.empty()) std::memcpy(b->h_ops, b->plan.ops.data(), b->plan.ops.size() * sizeof(CbOp));
     if (!PP.gates.empty()) std::memcpy(b->h_pgates, PP.gates.data(), PP.gates.size() * sizeof(double));
@@ -827,7 +828,6 @@ svb_status cb_create_with(svb_circuit_batch* proto, int MB, int threads, bool us
             pmost = std::max<uint64_t>(pmost, PP.phase_off[p + 1] - PP.phase_off[p]);
         b->pgrid = (unsigned)std::min<uint64_t>((uint64_t)pper * sms, pmost);
     }
-    if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail("stream", e);
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
         const cudaError_t le = cb_enqueue(b, b->stream);

@@ -545,6 +545,8 @@ struct Sim {
     bool have_circuit = false;
     cudaGraphExec_t graph = nullptr;
     cudaStream_t own_stream = nullptr;    // uploads of plans and capture of their graphs
+    cudaEvent_t uploaded = nullptr;       // behind the plan's copies
+    bool uploading = false;               // not yet seen to be complete
     svb_plan_info info{};
     // scratch
     MeasureScratch mscr;

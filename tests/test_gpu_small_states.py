@@ -87,3 +87,24 @@ def test_pauli_sums_of_amplitudes_whose_squares_overflow(n):
     t[0], t[1] = (0.5, 1, 0), (0.25, 1, 1)
     # <X_0> and <Y_0> of the pair (0, 1): 2 * 1e200 * 1e-190 and 2 * 1e200 * 2e-190
     assert abs(h.expectation(t) - (0.5 * 2e10 + 0.25 * 4e10)) <= 1e-4
+
+
+def test_a_small_circuit_captured_into_the_callers_graph(oracle):
+    """A run captured straight after its upload, replayed twice."""
+    import torch
+    from svsim_b200 import _native as nat
+    n = 8
+    g = circuits.random_matching_circuit(n, 6, seed=3)
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    h.set_engine(nat.ENGINE_PER_GATE)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    h.set_circuit(g)
+    with torch.cuda.graph(graph, stream=side):
+        h.run(side.cuda_stream)
+    with torch.cuda.stream(side):
+        graph.replay()
+        graph.replay()
+    side.synchronize()
+    re, im = h.get_state()
+    want = oracle.run(n, np.concatenate([g, g]))
+    assert np.array_equal(re, want[0]) and np.array_equal(im, want[1])
