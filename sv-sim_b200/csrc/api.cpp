@@ -12,6 +12,8 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 
 #include "bfly.h"
 #include "svb_internal.h"
@@ -614,14 +616,15 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         }
         engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
     }
-    if (engine == SVB_ENGINE_AUTO) {
+    const bool by_rule = engine == SVB_ENGINE_AUTO;
+    if (by_rule) {
         // Circuits of >= 12 qubits without SRN (which has no matrix) go to the tensor cores:
         // FP64 to the pair engine, FP32 to the fused engine (2x the staged engine at n = 24
         // and 30), or to butterflies where those are faster (FP32: unless a fusion width is
         // asked for); otherwise the staged engine, per-gate below its tile
         if (n >= PR_TILE_BITS && fusable(s->eops)) {
             engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
-            bfly = (engine == SVB_ENGINE_PAIRS || fusion == 0) && bfly_preferred(s->eops, n, s->precision);
+            bfly = (engine == SVB_ENGINE_PAIRS || fusion == 0) && bfly_candidate(s->eops, n, s->precision);
         } else {
             engine = (staged_supported(s->precision, M) && n >= M) ? SVB_ENGINE_STAGED : SVB_ENGINE_PER_GATE;
         }
@@ -660,12 +663,27 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     s->info.model_bytes = 2.0 * sb * sweeps;
     s->info.engine = engine;
     BfPlan B;
-    if (bfly && !plan_bfly(s->eops, n, s->precision, B, true)) {
-        if (s->engine_req == SVB_ENGINE_BUTTERFLY) {
+    bool pairs_planned = false;
+    if (bfly) {
+        // AUTO compares the FP64 plans of both forms, made on two host threads
+        std::thread helper;
+        bool ok = false;
+        const bool compare = by_rule && engine == SVB_ENGINE_PAIRS;
+        if (compare) {
+            try {
+                helper = std::thread([&] { ok = plan_bfly(s->eops, n, s->precision, B, true); });
+            } catch (const std::system_error&) {
+            }
+            pairs_planned = plan_pairs(s->eops, n, s->pairs, &s->mats);
+        }
+        if (helper.joinable()) helper.join();
+        else ok = plan_bfly(s->eops, n, s->precision, B, true);
+        bfly = ok && (!pairs_planned || bfly_cheaper(B, s->pairs, n));
+        if (bfly) s->pairs = PairPlan{};
+        if (!bfly && s->engine_req == SVB_ENGINE_BUTTERFLY) {
             set_error("svb_set_circuit: the butterfly planner rejected the circuit");
             return SVB_ERR_UNSUPPORTED;
         }
-        bfly = false;
     }
     if (bfly) {
         SVB_TRY(wait_plan_buf(s));
@@ -699,7 +717,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         // one read + write per pass, then the renormalisation (two reads, one write)
         s->info.moved_bytes = 2.0 * sb * (double)np + (np == 0 ? 0.0 : 3.0 * sb);
     } else if (engine == SVB_ENGINE_PAIRS) {
-        if (!plan_pairs(s->eops, n, s->pairs, &s->mats)) {
+        if (!pairs_planned && !plan_pairs(s->eops, n, s->pairs, &s->mats)) {
             set_error("svb_set_circuit: the pair planner rejected the circuit");
             return SVB_ERR_UNSUPPORTED;
         }

@@ -657,17 +657,24 @@ struct PassPlanner {
             if (start_reg[p] < 0) thr.push_back(p);
         const uint32_t low = ((1u << BF_COAL) - 1) << pack;
         auto in_low = [&](int p) { return col[p] && !(col[p] & ~low); };
+        uint16_t rslot[BF_TB], wslot[BF_TB];
+        for (int a = 0; a < BF_TB; a++) {
+            rslot[a] = slot(1u << thr[a]);
+            wslot[a] = slot(col[thr[a]]);
+        }
+        // the first choice of the highest value; no search beyond one that has all
+        const int most = 16 * loads + 16 * stores + 4 * reads + 4 * writes + (loads || stores);
         int best = -1, pick[3] = {0, 1, 2};
-        for (int a = 0; a < BF_TB; a++)
-            for (int b = a + 1; b < BF_TB; b++)
-                for (int c = 0; c < BF_TB; c++) {
+        for (int a = 0; a < BF_TB && best < most; a++)
+            for (int b = a + 1; b < BF_TB && best < most; b++)
+                for (int c = 0; c < BF_TB && best < most; c++) {
                     if (c == a || c == b) continue;
                     const int A = thr[a], B = thr[b], C = thr[c];
                     int v = 0;
                     if (loads && ((1u << A | 1u << B) == low)) v += 16;
                     if (stores && in_low(A) && in_low(B) && col[A] != col[B]) v += 16;
-                    if (reads && rank3(slot(1u << A), slot(1u << B), slot(1u << C))) v += 4;
-                    if (writes && rank3(slot(col[A]), slot(col[B]), slot(col[C]))) v += 4;
+                    if (reads && rank3(rslot[a], rslot[b], rslot[c])) v += 4;
+                    if (writes && rank3(wslot[a], wslot[b], wslot[c])) v += 4;
                     // lane 2 on the next lowest qubit: 128-byte runs
                     if ((loads && C == pack + BF_COAL) || (stores && col[C] == 1u << (pack + BF_COAL))) v += 1;
                     if (v > best) {
@@ -891,21 +898,16 @@ bool bfly_supported(const std::vector<EOp>& ops, int n, int precision)
     return true;
 }
 
-// Measured on one B200 against the tensor-core engines, GPU time of a run (set_circuit apart):
-//   phase-rich FP64: Fourier transform n = 16 / 20 / 25 68 / 136 / 4,679 us against 126 / 305 /
-//     13,527; half of the two-qubit gates phases or swaps, n = 16 / 20 / 25: 94 / 182 / 4,716 us
-//     against 96 / 192 / 5,979;
-//   other FP64 (random U3 + CX): n = 16 / 19 / 23 199 / 234 / 2,656 us against 193 / 224 / 2,639,
-//     n = 25 / 30 11.1 / 850 ms against 11.8 / 890: from n = 25 on, where a run is bound by the
-//     memory system's share that both have and the gates' FMAs that are half as many here;
-//   FP32: Fourier transform n = 16 / 20 / 25 86 / 125 / 3,122 us against 130 / 252 / 6,307, but
-//     the half-phases circuit 119 / 154 / 3,143 against 90 / 154 / 2,986 and random circuits
-//     240 / 283 / 7,274 (n = 16 / 19 / 25) against 156 / 199 / 5,566: FFMA2 on the CUDA cores
-//     against tcgen05, so only where phases outnumber the gates that need arithmetic.
-bool bfly_preferred(const std::vector<EOp>& raw, int n, int precision)
+// FP64: circuits with at least as many phases and swaps as CXs left, and others from 25 qubits
+// on with six gates a qubit or more; random U3 + CX circuits below 25 qubits take 0.94 (23
+// qubits, depth 25) to 1.5 (12 qubits, depth 2) of the blocks' time, from 25 qubits on those of
+// depth 2 to 4 1.04 to 1.38.
+// FP32: only where phases outnumber the gates that need arithmetic, FFMA2 on the CUDA cores
+// against tcgen05: Fourier transform of 13 / 16 / 20 / 28 qubits 0.80 / 0.67 / 0.50 / 0.45 of
+// the fused engine's time, half of the gates phases 0.8 to 1.4, random circuits 0.9 to 1.6.
+bool bfly_candidate(const std::vector<EOp>& raw, int n, int precision)
 {
     if (!bfly_supported(raw, n, precision)) return false;
-    if (precision == SVB_FP64 && n >= 25) return true;
     size_t phases = 0, swaps = 0, cx = 0, dense = 0;
     for (const EOp& e : shorten(raw)) {
         if (e.form == F_PP) phases++;
@@ -913,8 +915,37 @@ bool bfly_preferred(const std::vector<EOp>& raw, int n, int precision)
         else if (e.form == F_CX) cx++;
         else if (!form_is_diag(e.form)) dense++;
     }
-    if (precision == SVB_FP64) return phases + swaps >= cx && phases + swaps > 0;
+    if (precision == SVB_FP64) return (phases + swaps >= cx && phases + swaps > 0) || (n >= 25 && dense >= 6 * (size_t)n);
     return phases >= 2 * (dense + cx);
+}
+
+// Time of either plan by the counts of its parts, fitted to 526 circuits on one B200 (12 to 30
+// qubits; random, brickwork, mixed, Fourier transform; depth 2 to 30).  From 21 qubits on (two
+// tiles an SM and more) in us at 25 qubits, 1-2% off a run's time; below, the latency of one
+// tile, 10% off.  A gate costs a third of a two-qubit block, but a block takes in two gates and
+// more, so butterflies need some depth or phases.  At 25 qubits, of the blocks' time: random U3 +
+// CX of depth 2 / 4 / 10 / 30 1.2 / 1.07 / 0.98 / 0.94, brickwork 1.38 / 1.15 / 1.05 / 0.99, half
+// phases and swaps 1.09 / 0.94 / 0.85 / 0.8, Fourier transform 0.35.  Of the 316 candidates among
+// the circuits the choice was slower than the blocks by more than 2% on two (at most 2.6%) and
+// passed over up to 2% on three; butterflies for all of them were slower on 104 (up to 38%).
+bool bfly_cheaper(const BfPlan& b, const PairPlan& p, int n)
+{
+    // passes, relayouts, gates, scaled gates, register moves, phases, flushes; passes,
+    // relayouts, blocks, exchanges, lane permutations
+    struct Weights {
+        double b[7], p[5];
+    };
+    const Weights w = n > 20 ? Weights{{97, 32, 11.6, 17.7, 7.4, 8.9, 20}, {107, 80, 33.4, 3.2, 0}}
+                             : Weights{{7.8, 0.62, 0.28, 0.45, 0.48, 0.23, 0}, {7.4, 1.56, 0.34, 0.38, 0.3}};
+    size_t kind[BF_END + 1] = {0};
+    for (const BfOp& o : b.ops) kind[o.kind]++;
+    const size_t nb[7] = {b.passes.size(), b.rels.size(), kind[BF_ROT], kind[BF_SROT],
+                          kind[BF_CX],     kind[BF_DIAG], kind[BF_FLUSH]};
+    const size_t np[5] = {p.passes.size(), p.n_relayouts, p.n_blocks, p.n_swaps, p.n_lane_perms};
+    double tb = 0, tp = 0;
+    for (int i = 0; i < 7; i++) tb += w.b[i] * (double)nb[i];
+    for (int i = 0; i < 5; i++) tp += w.p[i] * (double)np[i];
+    return tb < tp;
 }
 
 std::vector<float> bfly_coefs32(const BfPlan& plan)

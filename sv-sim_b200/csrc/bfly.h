@@ -130,9 +130,11 @@ struct BfPlan {
 
 // whether every op is a unitary 2x2 matrix, a phase or a CX, and the state is big enough
 bool bfly_supported(const std::vector<EOp>& ops, int n, int precision);
-// Whether the engine is the faster one for the circuit (measured lines in bfly.cpp); implies
-// bfly_supported.
-bool bfly_preferred(const std::vector<EOp>& ops, int n, int precision);
+// Whether butterflies may be the faster form (implies bfly_supported): FP64 plans are then
+// compared, FP32 circuits take them.
+bool bfly_candidate(const std::vector<EOp>& ops, int n, int precision);
+// the comparison of the FP64 plans of one circuit
+bool bfly_cheaper(const BfPlan& b, const PairPlan& p, int n);
 // `tune` spends more host time on the choice of register qubits (1.5-3x the planning time).
 // False if a layout came out that the kernel cannot address, or a pass that does nothing of
 // what is left (neither has been seen; the caller then takes another engine).

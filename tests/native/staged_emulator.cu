@@ -798,3 +798,17 @@ extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, i
     for (uint64_t i = 0; i < dim; i++) { re[i] = sv[i].x; im[i] = sv[i].y; }
     return rc;
 }
+
+// Which form AUTO runs: 1 butterflies, 0 tensor-core blocks, -1 a gate with no lowering.
+extern "C" int emu_bfly_choice(uint32_t n, const svb_gate* gates, size_t n_gates, int precision)
+{
+    std::vector<EOp> eops;
+    for (size_t i = 0; i < n_gates; i++)
+        if (!lower_gate(gates[i], (int32_t)i, eops)) return -1;
+    if (!bfly_candidate(eops, (int)n, precision)) return 0;
+    if (precision != SVB_FP64) return 1;
+    BfPlan b;
+    PairPlan p;
+    if (!plan_bfly(eops, (int)n, precision, b, true)) return 0;
+    return !plan_pairs(eops, (int)n, p) || bfly_cheaper(b, p, (int)n);
+}

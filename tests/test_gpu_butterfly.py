@@ -35,6 +35,7 @@ def test_matches_the_per_gate_engine(n, precision, make):
     from svsim_b200 import _native as nat
     g = make(n, n)
     h = nat.Handle(n, 0, precision)
+    h.set_engine(nat.ENGINE_BUTTERFLY)
     ref = nat.Handle(n, 0, nat.SVB_FP64)
     ref.set_engine(nat.ENGINE_PER_GATE)
     h.set_circuit(g)

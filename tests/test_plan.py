@@ -568,3 +568,25 @@ def test_butterfly_plan_keeps_large_amplitudes_finite(emu, oracle, precision, fa
     err = np.sqrt(np.sum((re / factor - want[0]) ** 2 + (im / factor - want[1]) ** 2))
     norm = np.sqrt(np.sum(st ** 2))
     assert rc == 0 and err <= 8 * (2.2e-16 if precision == 0 else 1.2e-7) * np.sqrt(len(g) + 26) * norm
+
+
+def fourier(n):
+    gl = [G.U3(0.3 + 0.1 * q, 0.2, 0.1, q) for q in range(n)]
+    for i in range(n - 1, -1, -1):
+        gl += [G.H(i)] + [G.CU1(np.pi / (1 << (i - j)), j, i) for j in range(i - 1, -1, -1)]
+    return G.to_array(gl + [G.SWAP(q, n - 1 - q) for q in range(n // 2)])
+
+
+@pytest.mark.parametrize("make,n,depth,precision,form", [
+    # butterflies / blocks measured: 1.32, 1.1, 0.94, 0.95, 0.94; 1.38, 1.18, 1.05; 0.56, 0.37, 0.35
+    ("matching", 25, 2, 0, 0), ("matching", 28, 4, 0, 0), ("matching", 28, 30, 0, 1), ("matching", 30, 30, 0, 1),
+    ("matching", 30, 40, 0, 1), ("brickwork", 25, 2, 0, 0), ("brickwork", 28, 4, 0, 0), ("brickwork", 26, 10, 0, 0),
+    ("fourier", 16, 1, 0, 1), ("fourier", 24, 1, 0, 1), ("fourier", 25, 1, 0, 1), ("matching", 24, 25, 0, 0),
+    ("fourier", 16, 1, 1, 1), ("matching", 24, 25, 1, 0)])
+def test_default_form_is_the_faster_one(emu, make, n, depth, precision, form):
+    """AUTO's choice between blocks and butterflies, for circuits whose two times lie apart:
+    shallow random and brickwork circuits stay on blocks also from 25 qubits on."""
+    g = {"matching": lambda: circuits.random_matching_circuit(n, depth, seed=1),
+         "brickwork": lambda: circuits.brickwork_circuit(n, depth, seed=1), "fourier": lambda: fourier(n)}[make]()
+    assert emu.emu_bfly_choice(ctypes.c_uint32(n), ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)),
+                               precision) == form
