@@ -512,6 +512,7 @@ k_adj_stages(double2* __restrict__ psi, double2* __restrict__ lam, const AdjTile
 }
 
 // out = sum_t coef_t P_t psi
+template <bool FOUR>
 __global__ void __launch_bounds__(256)
 k_pauli_apply(const double2* __restrict__ psi, double2* __restrict__ out, uint64_t dim,
               const svb_pauli_term* __restrict__ terms, int n_terms)
@@ -520,8 +521,10 @@ k_pauli_apply(const double2* __restrict__ psi, double2* __restrict__ out, uint64
     for (int t = threadIdx.x; t < n_terms; t += blockDim.x) sterms[t] = terms[t];
     __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += PAULI_U * stride)
-        pauli_apply(psi, out, i, stride, dim, sterms, n_terms);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += (FOUR ? PAULI_U : 1) * stride) {
+        if (FOUR) pauli_apply(psi, out, i, stride, dim, sterms, n_terms);
+        else out[i] = pauli_apply_one(psi, i, sterms, n_terms);
+    }
 }
 
 __global__ void __launch_bounds__(256)
@@ -981,11 +984,12 @@ extern "C" svb_status svb_adjoint(svb_sim* s, const svb_gate* gates, const svb_p
     if ((err = cudaMemcpyAsync(A.final_state.p, s->state, sbytes, cudaMemcpyDeviceToDevice)) != cudaSuccess)
         return fail(err, "final state copy");
     // lambda = H psi, energy = Re <psi|lambda>
-    if (n_terms)
-        k_pauli_apply<<<(unsigned)std::min<uint64_t>((dim + 256 * PAULI_U - 1) / (256 * PAULI_U), 148 * 16), 256,
-                        n_terms * sizeof(svb_pauli_term)>>>(
+    if (n_terms) {
+        const bool four = pauli_by_four(dim, (int)n_terms, PAULI_APPLY_BITS);
+        const unsigned grid = four ? (unsigned)std::min<uint64_t>(dim / (256 * PAULI_U), 148 * 16) : adj_grid(dim);
+        (four ? k_pauli_apply<true> : k_pauli_apply<false>)<<<grid, 256, n_terms * sizeof(svb_pauli_term)>>>(
             static_cast<const double2*>(s->state), lam, dim, dterms, (int)n_terms);
-    else
+    } else
         err = cudaMemset(lam, 0, sbytes);
     k_inner_re<<<ADJ_BLOCKS, 256>>>(static_cast<const double2*>(s->state), lam, dim, partial + eoff);
     k_reduce_rows<<<1, 32>>>(partial + eoff, ADJ_BLOCKS, ADJ_BLOCKS, 1, results + slots.size());

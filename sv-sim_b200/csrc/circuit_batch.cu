@@ -191,6 +191,51 @@ __device__ __forceinline__ double cb_warp_sum(double v)
     return v;
 }
 
+// partial energies, one warp per chunk
+template <typename T, bool FOUR>
+__device__ __forceinline__ void cb_chunk_energies(const CbArgs& A)
+{
+    using V = typename VecOf<T>::type;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < A.n_chunks; k += warps) {
+        const CbCircuit C = A.circ[A.chunk_circ[k]];
+        const uint64_t dim = 1ull << C.n;
+        const uint64_t start = (uint64_t)(k - C.chunk_begin) * CB_CHUNK;
+        const uint64_t end = start + CB_CHUNK < dim ? start + CB_CHUNK : dim;
+        const V* sv = static_cast<const V*>(A.pool) + C.state_off;
+        const svb_pauli_term* terms = A.terms + C.term_begin;
+        const int n_terms = (int)(C.term_end - C.term_begin);
+        double acc = 0.0;
+        if (FOUR && pauli_by_four(dim, n_terms, PAULI_CHUNK_BITS))
+            for (uint64_t i = start + lane; i < end; i += 32 * PAULI_U)
+                acc += pauli_energy<T>(sv, i, 32, end, terms, n_terms);
+        else
+            for (uint64_t i = start + lane; i < end; i += 32) acc += pauli_energy_one<T>(sv, i, terms, n_terms);
+        acc = cb_warp_sum(acc);
+        if (lane == 0) A.partial[k] = acc;
+    }
+}
+
+// one warp per circuit over its chunks in order
+__device__ __forceinline__ void cb_sum_energies(const CbArgs& A)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < (uint32_t)A.n_circ; c += warps) {
+        const CbCircuit C = A.circ[c];
+        if (C.term_end == C.term_begin) {
+            if (lane == 0) A.energy[c] = 0.0;
+            continue;
+        }
+        const uint64_t nch = ((1ull << C.n) + CB_CHUNK - 1) / CB_CHUNK;
+        double s = 0.0;
+        for (uint64_t k = lane; k < nch; k += 32) s += A.partial[C.chunk_begin + k];
+        s = cb_warp_sum(s);
+        if (lane == 0) A.energy[c] = s;
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512) k_cbatch(CbArgs A)
 {
@@ -234,38 +279,24 @@ __global__ void __launch_bounds__(512) k_cbatch(CbArgs A)
         cb_grid_barrier(A.barrier, target);
     }
     if (A.n_chunks == 0) return;
-    // energies: one warp per chunk, then one warp per circuit over its chunks in order
-    const int lane = threadIdx.x & 31;
-    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    for (uint32_t k = wid; k < A.n_chunks; k += warps) {
-        const CbCircuit C = A.circ[A.chunk_circ[k]];
-        const uint64_t dim = 1ull << C.n;
-        const uint64_t start = (uint64_t)(k - C.chunk_begin) * CB_CHUNK;
-        const uint64_t end = start + CB_CHUNK < dim ? start + CB_CHUNK : dim;
-        const V* sv = pool + C.state_off;
-        double acc = 0.0;
-        const int n_terms = (int)(C.term_end - C.term_begin);
-        if (n_terms > 0)
-            for (uint64_t i = start + lane; i < end; i += 32 * PAULI_U)
-                acc += pauli_energy<T>(sv, i, 32, end, A.terms + C.term_begin, n_terms);
-        acc = cb_warp_sum(acc);
-        if (lane == 0) A.partial[k] = acc;
-    }
+    cb_chunk_energies<T, false>(A);
     target += gridDim.x;
     cb_grid_barrier(A.barrier, target);
-    for (uint32_t c = wid; c < (uint32_t)A.n_circ; c += warps) {
-        const CbCircuit C = A.circ[c];
-        if (C.term_end == C.term_begin) {
-            if (lane == 0) A.energy[c] = 0.0;
-            continue;
-        }
-        const uint64_t nch = ((1ull << C.n) + CB_CHUNK - 1) / CB_CHUNK;
-        double s = 0.0;
-        for (uint64_t k = lane; k < nch; k += 32) s += A.partial[C.chunk_begin + k];
-        s = cb_warp_sum(s);
-        if (lane == 0) A.energy[c] = s;
-    }
+    cb_sum_energies(A);
+}
+
+// The energies of a batch in which some circuit's go four amplitudes at a time, after k_cbatch
+// (which then has no chunks): in one kernel with the passes that form's registers (84 instead of
+// 50) halved the CTAs an SM held during the passes (512 circuits of 14 qubits, a layer and one
+// string each: 0.80 -> 1.15 ms).
+template <typename T>
+__global__ void __launch_bounds__(256) k_cb_energies(CbArgs A)
+{
+    cb_chunk_energies<T, true>(A);
+}
+__global__ void __launch_bounds__(256) k_cb_energy_sums(CbArgs A)
+{
+    cb_sum_energies(A);
 }
 
 template <typename T>
@@ -357,6 +388,7 @@ struct CbPlan {
     std::vector<CbItem> items;
     std::vector<uint32_t> phase_off;
     std::vector<uint32_t> chunk_circ;
+    bool by_four = false;                // energies by k_cb_energies
     uint64_t pool_amps = 0;
     double moved_bytes = 0;
     CbPairPlan pairs;
@@ -600,6 +632,7 @@ bool cb_build_plan(const svb_circuit_batch* b, const svb_gate* gates, int MB, bo
             const uint64_t nch = ((1ull << n) + CB_CHUNK - 1) / CB_CHUNK;
             for (uint64_t k = 0; k < nch; k++) plan.chunk_circ.push_back(c);
             chunks += (uint32_t)nch;
+            plan.by_four |= pauli_by_four(1ull << n, (int)(C.term_end - C.term_begin), PAULI_CHUNK_BITS);
         }
         plan.pool_amps += 1ull << n;
         plan.circ.push_back(C);
@@ -695,10 +728,18 @@ cudaError_t cb_launch(svb_circuit_batch* b, cudaStream_t s)
     a.barrier = b->d_bar;
     a.n_phases = (int)b->plan.phase_off.size() - 1;
     a.n_circ = (int)b->n_circ;
-    a.n_chunks = (uint32_t)b->plan.chunk_circ.size();
+    const uint32_t chunks = (uint32_t)b->plan.chunk_circ.size();
+    a.n_chunks = b->plan.by_four ? 0 : chunks;
     a.pad = 0;
     void* args[] = {&a};
-    return cudaLaunchCooperativeKernel((const void*)k_cbatch<T>, dim3(b->grid), dim3(b->threads), args, b->smem, s);
+    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_cbatch<T>, dim3(b->grid), dim3(b->threads), args, b->smem, s);
+    if (e == cudaSuccess && b->plan.by_four) {
+        a.n_chunks = chunks;
+        k_cb_energies<T><<<std::min<unsigned>((chunks + 7) / 8, 148 * 16), 256, 0, s>>>(a);
+        k_cb_energy_sums<<<std::min<unsigned>((b->n_circ + 7) / 8, 148 * 4), 256, 0, s>>>(a);
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t cb_launch_pairs(svb_circuit_batch* b, cudaStream_t s)

@@ -784,7 +784,7 @@ k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uin
     if (lane == 0) out[shot] = result;
 }
 
-template <typename T>
+template <typename T, bool FOUR>
 __global__ void __launch_bounds__(256)
 k_pauli_expect(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim,
                const svb_pauli_term* __restrict__ terms, int n_terms, double* __restrict__ partial)
@@ -795,8 +795,9 @@ k_pauli_expect(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim,
     __syncthreads();
     double acc = 0.0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += PAULI_U * stride)
-        acc += pauli_energy<T>(sv, i, stride, dim, sterms, n_terms);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < dim; i += (FOUR ? PAULI_U : 1) * stride)
+        acc += FOUR ? pauli_energy<T>(sv, i, stride, dim, sterms, n_terms)
+                    : pauli_energy_one<T>(sv, i, sterms, n_terms);
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
@@ -950,8 +951,12 @@ cudaError_t expectation_device(const void* state, int n, const svb_pauli_term* d
     using V = typename VecOf<T>::type;
     const uint64_t dim = 1ull << n;
     const size_t smem = sizeof(svb_pauli_term) * (size_t)n_terms;
-    k_pauli_expect<T><<<REDUCE_BLOCKS, 256, smem, s>>>(static_cast<const V*>(state), dim, d_terms,
-                                                        n_terms, d_partial);
+    if (pauli_by_four(dim, n_terms, PAULI_STATE_BITS))
+        k_pauli_expect<T, true><<<REDUCE_BLOCKS, 256, smem, s>>>(static_cast<const V*>(state), dim, d_terms,
+                                                                  n_terms, d_partial);
+    else
+        k_pauli_expect<T, false><<<REDUCE_BLOCKS, 256, smem, s>>>(static_cast<const V*>(state), dim, d_terms,
+                                                                   n_terms, d_partial);
     k_sum_partials<<<1, 32, 0, s>>>(d_partial, REDUCE_BLOCKS, d_out);
     return cudaGetLastError();
 }

@@ -108,3 +108,34 @@ def test_a_small_circuit_captured_into_the_callers_graph(oracle):
     re, im = h.get_state()
     want = oracle.run(n, np.concatenate([g, g]))
     assert np.array_equal(re, want[0]) and np.array_equal(im, want[1])
+
+
+@pytest.mark.parametrize("n,count", [(7, 4), (8, 3), (8, 4), (8, 300), (16, 5), (17, 3), (17, 4), (18, 4), (19, 3), (19, 4),
+                                     (20, 9)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_pauli_sums_on_both_sides_of_the_lines_between_their_forms(oracle, n, count, precision):
+    """One amplitude at a time and four at a time, by svb_expectation (19 qubits and 4 terms), in
+    the adjoint (17) and in a batch, whose circuits then differ in their form (8): the oracle's
+    sum, to 1e-14 a term of coefficient 1 (FP32: the state's rounding)."""
+    from svsim_b200 import _native as nat
+    rng = np.random.default_rng(n * 100 + count)
+    g = circuits.random_matching_circuit(n, 3, seed=n)
+    t = random_terms(n, count, rng)
+    re, im = oracle.run(n, g)
+    want = oracle.expectation(n, re, im, t)
+    bound = (1e-14 if precision == 0 else 2e-6) * float(np.sum(np.abs(t["coef"])))
+    h = nat.Handle(n, 0, precision)
+    h.set_circuit(g)
+    h.run()
+    assert abs(h.expectation(t) - want) <= bound
+    small = circuits.random_matching_circuit(3, 2, seed=1)
+    ts = random_terms(3, 5, rng)
+    b = nat.CircuitBatch([(n, g), (3, small), (2, small[:0])], [t, ts, None], precision=precision)
+    e = b.run()
+    assert abs(e[0] - want) <= bound and e[2] == 0.0
+    assert abs(e[1] - oracle.expectation(3, *oracle.run(3, small), ts)) <= (1e-13 if precision == 0 else 1e-5)
+    if precision == 0:
+        binding = np.zeros(len(g), dtype=G.PARAM_DTYPE)
+        binding["idx"] = -1
+        ea, _ = h.adjoint(g, binding, 0, t)
+        assert abs(ea - want) <= bound
