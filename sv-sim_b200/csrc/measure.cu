@@ -676,6 +676,12 @@ k_cdf_fill(const uint64_t* __restrict__ entry, uint64_t nblocks, uint64_t nsuper
 // chunk c's sum and whether it has no tie, NaN or inf.  The 16 loads a lane are in flight
 // together and the 16 sums share one exchange (31 shuffles a lane instead of 160).
 constexpr int SHOT_GROUP = 16;
+// A state of few chunks is walked chunk by chunk: its shots lie a few chunks in, where a group's
+// 16 loads and the kernel's 63 registers (34 without) only cost when there are many shots.
+// svb_measure, chunks / groups in us, FP32 random state: 50,000 shots on 8, 10, 11, 12 qubits
+// 332 / 451, 579 / 788, 865 / 1,125, 1,429 (chunks before groups) / 1,415; 1,000 shots on 10 and
+// 11 qubits (FP64, uniform state) 81 / 73, 96 / 82.
+constexpr bool shot_groups(int n, uint32_t shots) { return n >= 12 || (n >= 10 && shots <= 2048); }
 template <typename T>
 __device__ __forceinline__ uint64_t group_units(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim,
                                                 uint64_t first, uint32_t code, int lane, bool* fits)
@@ -715,7 +721,7 @@ __device__ __forceinline__ uint64_t group_units(const typename VecOf<T>::type* _
 // 94 us while such a group was added element by element throughout, 34 us now (n = 16; 30 at
 // n = 23).  Shots with no such j (r >= S_{2^n}, r < 0 or
 // NaN) give 0 as in the reference.
-template <typename T>
+template <typename T, bool GROUPS>
 __global__ void __launch_bounds__(256)
 k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uint64_t nblocks,
                const double* __restrict__ start, const double* __restrict__ uniforms, uint32_t shots,
@@ -744,7 +750,7 @@ k_sample_exact(const typename VecOf<T>::type* __restrict__ sv, uint64_t dim, uin
             uint64_t m = 0;
             const uint32_t code = binade_of(s, &m);
             int f = cur;                 // chunk to add element by element
-            if (code != 0) {
+            if (GROUPS && code != 0) {
                 const int g = cur & ~(SHOT_GROUP - 1);
                 if (code != have || g != group) {
                     units = group_units<T>(sv, dim, base + (uint64_t)g * 32, code, lane, &fits);
@@ -919,7 +925,10 @@ cudaError_t measure_device(const void* state, int n, const double* d_uniforms, u
     // 6. samples
     if (shots > 0) {
         const unsigned sblocks = (unsigned)(((uint64_t)shots * 32 + 255) / 256);
-        k_sample_exact<T><<<sblocks, 256, 0, s>>>(sv, dim, L.nblocks, start, d_uniforms, shots, d_samples);
+        if (shot_groups(n, shots))
+            k_sample_exact<T, true><<<sblocks, 256, 0, s>>>(sv, dim, L.nblocks, start, d_uniforms, shots, d_samples);
+        else
+            k_sample_exact<T, false><<<sblocks, 256, 0, s>>>(sv, dim, L.nblocks, start, d_uniforms, shots, d_samples);
     }
     cudaError_t e = cudaSuccess;
     if (d_total)

@@ -206,3 +206,20 @@ def test_edges_with_ties_of_both_parities(oracle, n, share):
     h = nat.Handle(n, 0, nat.SVB_FP64)
     h.set_state(re, im)
     check_state(oracle, h, n, rng)
+
+
+@pytest.mark.parametrize("n", [9, 10, 11, 12])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_few_and_many_shots_of_small_states(oracle, n, precision):
+    """Shots walked chunk by chunk and by groups of chunks: below 10 qubits, from 12 on, and in
+    between by the number of shots (2,048)."""
+    nat = native()
+    h = nat.Handle(n, 0, precision)
+    h.set_circuit(circuits.random_matching_circuit(n, 4, seed=n))
+    h.run()
+    rng = np.random.default_rng(n)
+    check_state(oracle, h, n, rng)
+    re, im = h.get_state()
+    u = np.concatenate([edge_uniforms(sequential_scan(re, im), rng), rng.random(2048)])
+    got, _ = h.measure(u)
+    assert np.array_equal(got, oracle.measure(n, re, im, u)[0])
