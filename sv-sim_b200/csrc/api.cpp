@@ -755,7 +755,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         for (const EOp& e : s->eops)
             moved += (e.form == F_CX || (form_is_diag(e.form) && e.form != F_DIAG)) ? sb : 2.0 * sb;
         s->info.moved_bytes = moved;
-        if (n <= SMALL_QUBITS && !s->eops.empty()) {
+        if (n <= SMALL_QUBITS && s->eops.size() >= SMALL_MIN_OPS) {
             // one launch: the state goes through shared memory once
             const size_t ob = s->eops.size() * sizeof(SmallOp), mb = s->mats.size() * sizeof(Mat4);
             std::vector<unsigned char> host(ob + mb);
@@ -780,8 +780,9 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             s->info.moved_bytes = 2.0 * sb;
         }
     }
-    SVB_CUDA(cudaEventRecord(s->uploaded, s->own_stream), "cudaEventRecord");
-    s->uploading = true;
+    // sweeps of single gates have their matrices in the launches
+    s->uploading = engine != SVB_ENGINE_PER_GATE || s->small_ops;
+    if (s->uploading) SVB_CUDA(cudaEventRecord(s->uploaded, s->own_stream), "cudaEventRecord");
     s->have_circuit = true;
     return SVB_OK;
 }

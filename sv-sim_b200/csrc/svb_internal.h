@@ -398,6 +398,10 @@ template <typename T>
 cudaError_t launch_eop(void* state, int n, const EOp& op, cudaStream_t s);
 // the per-gate engine on a state of at most SMALL_QUBITS qubits: all ops in one launch
 constexpr int SMALL_QUBITS = 12;         // 64 KiB of FP64 state in shared memory
+// A single op is launched by itself: the list's upload costs 4-5 us a circuit (upload and run of
+// one gate 11.5 us against 17, of two 14 against 17, three 17 and 17.5), a run is no shorter (of
+// one gate on 6 / 12 qubits 4.4 / 4.6 us against 4.9 / 6.6, of two 6.9 / 7.4 against 5.0 / 7.4).
+constexpr size_t SMALL_MIN_OPS = 2;
 struct alignas(16) SmallOp {             // 80 bytes
     double m[8];
     uint8_t form, q, c, pad;
