@@ -608,7 +608,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             return SVB_ERR_UNSUPPORTED;
         }
     }
-    bool bfly = engine == SVB_ENGINE_BUTTERFLY;
+    bool bfly = engine == SVB_ENGINE_BUTTERFLY, compare = false;
     if (bfly) {
         if (!bfly_supported(s->eops, n, s->precision)) {
             set_error("svb_set_circuit: butterflies need >= 12 qubits (13 in FP32) and no SRN or R");
@@ -616,15 +616,18 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         }
         engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
     }
-    const bool by_rule = engine == SVB_ENGINE_AUTO;
-    if (by_rule) {
+    if (engine == SVB_ENGINE_AUTO) {
         // Circuits of >= 12 qubits without SRN (which has no matrix) go to the tensor cores:
         // FP64 to the pair engine, FP32 to the fused engine (2x the staged engine at n = 24
         // and 30), or to butterflies where those are faster (FP32: unless a fusion width is
         // asked for); otherwise the staged engine, per-gate below its tile
         if (n >= PR_TILE_BITS && fusable(s->eops)) {
             engine = s->precision == SVB_FP64 ? SVB_ENGINE_PAIRS : SVB_ENGINE_FUSED;
-            bfly = (engine == SVB_ENGINE_PAIRS || fusion == 0) && bfly_candidate(s->eops, n, s->precision);
+            if (engine == SVB_ENGINE_PAIRS || fusion == 0) {
+                const BfChoice choice = bfly_choice(s->eops, n, s->precision);
+                bfly = choice != BfChoice::BLOCKS;
+                compare = choice == BfChoice::COMPARE;
+            }
         } else {
             engine = (staged_supported(s->precision, M) && n >= M) ? SVB_ENGINE_STAGED : SVB_ENGINE_PER_GATE;
         }
@@ -665,10 +668,9 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     BfPlan B;
     bool pairs_planned = false;
     if (bfly) {
-        // AUTO compares the FP64 plans of both forms, made on two host threads
+        // the FP64 plans of both forms to compare, made on two host threads
         std::thread helper;
         bool ok = false;
-        const bool compare = by_rule && engine == SVB_ENGINE_PAIRS;
         if (compare) {
             try {
                 helper = std::thread([&] { ok = plan_bfly(s->eops, n, s->precision, B, true); });
@@ -678,7 +680,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         }
         if (helper.joinable()) helper.join();
         else ok = plan_bfly(s->eops, n, s->precision, B, true);
-        bfly = ok && (!pairs_planned || bfly_cheaper(B, s->pairs, n));
+        bfly = ok && (!pairs_planned || bfly_cheaper(B, s->pairs));
         if (bfly) s->pairs = PairPlan{};
         if (!bfly && s->engine_req == SVB_ENGINE_BUTTERFLY) {
             set_error("svb_set_circuit: the butterfly planner rejected the circuit");

@@ -898,16 +898,22 @@ bool bfly_supported(const std::vector<EOp>& ops, int n, int precision)
     return true;
 }
 
-// FP64: circuits with at least as many phases and swaps as CXs left, and others from 25 qubits
-// on with six gates a qubit or more; random U3 + CX circuits below 25 qubits take 0.94 (23
-// qubits, depth 25) to 1.5 (12 qubits, depth 2) of the blocks' time, from 25 qubits on those of
-// depth 2 to 4 1.04 to 1.38.
+// FP64, by the counts of the shortened circuit: the estimate is the logarithm of butterflies'
+// time over the blocks', fitted to the circuits below with as many phases and swaps as CXs (off
+// by 0.19, one sigma).  Where it is clear one form is planned, since a second plan takes as long
+// as 1 to 4 runs up to 20 qubits (Fourier transform of 16 qubits, upload and run 440 us, with
+// both plans 550) and 7% of a run at 25.  Up to 20 qubits the estimate decides alone: of 164 such
+// circuits it took butterflies on 14 whose runs are 2-19% slower, 1 to 7 us, and whose planning
+// is 10 to 40 us shorter, and passed over 5-14% on three; butterflies for all of them were slower
+// on 37, by up to 32%.  Circuits of more CXs take 0.94 (23 qubits, depth 25) to 1.5 (12 qubits,
+// depth 2) of the blocks' time below 25 qubits, and from 25 on 1.04 to 1.38 at depth 2 to 4.
 // FP32: only where phases outnumber the gates that need arithmetic, FFMA2 on the CUDA cores
 // against tcgen05: Fourier transform of 13 / 16 / 20 / 28 qubits 0.80 / 0.67 / 0.50 / 0.45 of
-// the fused engine's time, half of the gates phases 0.8 to 1.4, random circuits 0.9 to 1.6.
-bool bfly_candidate(const std::vector<EOp>& raw, int n, int precision)
+// the fused engine's time, ten layers of controlled phases 0.55 to 0.83, half of the gates phases
+// 0.8 to 1.4, random circuits 0.9 to 1.6.
+BfChoice bfly_choice(const std::vector<EOp>& raw, int n, int precision)
 {
-    if (!bfly_supported(raw, n, precision)) return false;
+    if (!bfly_supported(raw, n, precision)) return BfChoice::BLOCKS;
     size_t phases = 0, swaps = 0, cx = 0, dense = 0;
     for (const EOp& e : shorten(raw)) {
         if (e.form == F_PP) phases++;
@@ -915,36 +921,40 @@ bool bfly_candidate(const std::vector<EOp>& raw, int n, int precision)
         else if (e.form == F_CX) cx++;
         else if (!form_is_diag(e.form)) dense++;
     }
-    if (precision == SVB_FP64) return (phases + swaps >= cx && phases + swaps > 0) || (n >= 25 && dense >= 6 * (size_t)n);
-    return phases >= 2 * (dense + cx);
+    if (precision == SVB_FP32) return phases >= 2 * (dense + cx) ? BfChoice::BUTTERFLIES : BfChoice::BLOCKS;
+    if (phases + swaps == 0 || phases + swaps < cx)
+        return n >= 25 && dense >= 6 * (size_t)n ? BfChoice::COMPARE : BfChoice::BLOCKS;
+    const double two = (double)(phases + swaps + cx);
+    const double estimate = -0.82 + (0.28 * (double)dense + 0.78 * (double)cx + 0.105 * n) / two;
+    if (n <= 20) return estimate < 0 ? BfChoice::BUTTERFLIES : BfChoice::BLOCKS;
+    return estimate < -0.2 ? BfChoice::BUTTERFLIES : (estimate > 0.05 ? BfChoice::BLOCKS : BfChoice::COMPARE);
 }
 
-// Time of either plan by the counts of its parts, fitted to 526 circuits on one B200 (12 to 30
-// qubits; random, brickwork, mixed, Fourier transform; depth 2 to 30).  From 21 qubits on (two
-// tiles an SM and more) in us at 25 qubits, 1-2% off a run's time; below, the latency of one
-// tile, 10% off.  A gate costs a third of a two-qubit block, but a block takes in two gates and
-// more, so butterflies need some depth or phases.  At 25 qubits, of the blocks' time: random U3 +
-// CX of depth 2 / 4 / 10 / 30 1.2 / 1.07 / 0.98 / 0.94, brickwork 1.38 / 1.15 / 1.05 / 0.99, half
-// phases and swaps 1.09 / 0.94 / 0.85 / 0.8, Fourier transform 0.35.  Of the 316 candidates among
-// the circuits the choice was slower than the blocks by more than 2% on two (at most 2.6%) and
-// passed over up to 2% on three; butterflies for all of them were slower on 104 (up to 38%).
-bool bfly_cheaper(const BfPlan& b, const PairPlan& p, int n)
+// Time of either plan by the counts of its parts in us at 25 qubits (from 21 on there are two
+// tiles an SM and more), fitted to 188 circuits of 25 to 30 qubits on one B200 (random,
+// brickwork, mixed, Fourier transform; depth 2 to 30): 1-2% off a run's time.  A gate costs a
+// third of a two-qubit block, but a block takes in two gates and more, so butterflies need some
+// depth or phases.  At 25 qubits, of the blocks' time: random U3 + CX of depth 2 / 4 / 10 / 30
+// 1.2 / 1.07 / 0.98 / 0.94, brickwork 1.38 / 1.15 / 1.05 / 0.99, half phases and swaps 1.09 /
+// 0.94 / 0.85 / 0.8, Fourier transform 0.35.  Of 227 circuits of 21 to 30 qubits the comparison
+// was wrong by more than 1% on three (at most 1.4%) and passed over up to 2% on three;
+// butterflies for all of them were slower on 78 (up to 38%).
+bool bfly_cheaper(const BfPlan& b, const PairPlan& p)
 {
     // passes, relayouts, gates, scaled gates, register moves, phases, flushes; passes,
-    // relayouts, blocks, exchanges, lane permutations
+    // relayouts, blocks, exchanges (a lane permutation's share did not show)
     struct Weights {
-        double b[7], p[5];
+        double b[7], p[4];
     };
-    const Weights w = n > 20 ? Weights{{97, 32, 11.6, 17.7, 7.4, 8.9, 20}, {107, 80, 33.4, 3.2, 0}}
-                             : Weights{{7.8, 0.62, 0.28, 0.45, 0.48, 0.23, 0}, {7.4, 1.56, 0.34, 0.38, 0.3}};
+    const Weights w = {{97, 32, 11.6, 17.7, 7.4, 8.9, 20}, {107, 80, 33.4, 3.2}};
     size_t kind[BF_END + 1] = {0};
     for (const BfOp& o : b.ops) kind[o.kind]++;
     const size_t nb[7] = {b.passes.size(), b.rels.size(), kind[BF_ROT], kind[BF_SROT],
                           kind[BF_CX],     kind[BF_DIAG], kind[BF_FLUSH]};
-    const size_t np[5] = {p.passes.size(), p.n_relayouts, p.n_blocks, p.n_swaps, p.n_lane_perms};
+    const size_t np[4] = {p.passes.size(), p.n_relayouts, p.n_blocks, p.n_swaps};
     double tb = 0, tp = 0;
     for (int i = 0; i < 7; i++) tb += w.b[i] * (double)nb[i];
-    for (int i = 0; i < 5; i++) tp += w.p[i] * (double)np[i];
+    for (int i = 0; i < 4; i++) tp += w.p[i] * (double)np[i];
     return tb < tp;
 }
 

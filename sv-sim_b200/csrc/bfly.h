@@ -130,11 +130,11 @@ struct BfPlan {
 
 // whether every op is a unitary 2x2 matrix, a phase or a CX, and the state is big enough
 bool bfly_supported(const std::vector<EOp>& ops, int n, int precision);
-// Whether butterflies may be the faster form (implies bfly_supported): FP64 plans are then
-// compared, FP32 circuits take them.
-bool bfly_candidate(const std::vector<EOp>& ops, int n, int precision);
+// The faster form by a circuit's counts, where those tell (butterflies only if bfly_supported).
+enum class BfChoice { BLOCKS, BUTTERFLIES, COMPARE };
+BfChoice bfly_choice(const std::vector<EOp>& ops, int n, int precision);
 // the comparison of the FP64 plans of one circuit
-bool bfly_cheaper(const BfPlan& b, const PairPlan& p, int n);
+bool bfly_cheaper(const BfPlan& b, const PairPlan& p);
 // `tune` spends more host time on the choice of register qubits (1.5-3x the planning time).
 // False if a layout came out that the kernel cannot address, or a pass that does nothing of
 // what is left (neither has been seen; the caller then takes another engine).

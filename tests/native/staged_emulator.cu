@@ -805,10 +805,10 @@ extern "C" int emu_bfly_choice(uint32_t n, const svb_gate* gates, size_t n_gates
     std::vector<EOp> eops;
     for (size_t i = 0; i < n_gates; i++)
         if (!lower_gate(gates[i], (int32_t)i, eops)) return -1;
-    if (!bfly_candidate(eops, (int)n, precision)) return 0;
-    if (precision != SVB_FP64) return 1;
+    const BfChoice choice = bfly_choice(eops, (int)n, precision);
+    if (choice != BfChoice::COMPARE) return choice == BfChoice::BUTTERFLIES;
     BfPlan b;
     PairPlan p;
     if (!plan_bfly(eops, (int)n, precision, b, true)) return 0;
-    return !plan_pairs(eops, (int)n, p) || bfly_cheaper(b, p, (int)n);
+    return !plan_pairs(eops, (int)n, p) || bfly_cheaper(b, p);
 }
