@@ -431,8 +431,7 @@ svb_status svb_create(uint32_t n_qubits, int device, int precision, svb_sim** ou
     if (e != cudaSuccess) { delete s; return cuda_fail(e, "cudaMalloc(state)"); }
     e = cudaMalloc(&s->d_small, 64 * sizeof(double));
     if (e != cudaSuccess) { cudaFree(s->state); delete s; return cuda_fail(e, "cudaMalloc"); }
-    e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->uploaded, cudaEventDisableTiming);
+    e = cudaEventCreateWithFlags(&s->uploaded, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->plan_read, cudaEventDisableTiming);
     if (e == cudaSuccess)
         e = dispatch_prec(precision, [&](auto t) {
@@ -456,7 +455,7 @@ svb_status svb_destroy(svb_sim* s)
     free_scratch(s);
     cudaFree(s->state);
     cudaFree(s->d_small);
-    if (s->own_stream) cudaStreamDestroy(s->own_stream);
+    if (s->capture_stream) cudaStreamDestroy(s->capture_stream);
     if (s->uploaded) cudaEventDestroy(s->uploaded);
     if (s->plan_read) cudaEventDestroy(s->plan_read);
     delete s;
@@ -531,15 +530,15 @@ std::array<uint64_t, 4> structure_key(const Sim* s, const std::vector<EOp>& eops
 }
 
 // A new device buffer of a plan with the host's values in it, of at least `least` of them.
-// The copy is on the handle's own stream, behind no other handle's work.  It can return before
-// it has reached the device: svb_run makes its stream wait for s->uploaded.  (Four copies of
-// 1.6 MB in all: 72 us with the event, 96 by cudaMemcpy, 92 with a wait for the stream.)
+// A copy from pageable memory can return before it has reached the device: svb_run makes its
+// stream wait for s->uploaded.  (Four copies of 1.6 MB in all: 72 us with the event, 96 by
+// cudaMemcpy, 115 with a wait for the stream.)
 template <typename T>
 svb_status upload(Sim* s, T** dst, const std::vector<T>& v, size_t least = 1)
 {
     SVB_CUDA(cudaMalloc(dst, std::max(least, v.size()) * sizeof(T)), "cudaMalloc(plan)");
     if (!v.empty())
-        SVB_CUDA(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s->own_stream),
+        SVB_CUDA(cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, nullptr),
                  "plan upload");
     return SVB_OK;
 }
@@ -689,7 +688,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     }
     if (bfly) {
         SVB_TRY(wait_plan_buf(s));
-        SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly, s->own_stream), "plan upload");
+        SVB_CUDA(upload_bfly(B, s->precision, s->plan_buf, s->dbfly), "plan upload");
         s->bfly = true;
         s->info.n_passes = B.passes.size();
         s->info.tile_bits = B.tile_bits;
@@ -708,7 +707,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         SVB_TRY(upload(s, &s->dfused.gates, F.gates, 4));
         if (!F.passes6.empty()) SVB_TRY(upload(s, &s->dfused.passes6, F.passes6));
         SVB_CUDA(cudaMalloc(&s->dfused.err, sizeof(int)), "cudaMalloc(flag)");
-        SVB_CUDA(cudaMemsetAsync(s->dfused.err, 0, sizeof(int), s->own_stream), "cudaMemset");
+        SVB_CUDA(cudaMemsetAsync(s->dfused.err, 0, sizeof(int), nullptr), "cudaMemset");
         SVB_CUDA(cudaMalloc(&s->dfused.norm_partial, REDUCE_BLOCKS * sizeof(double)), "cudaMalloc(norm)");
         const size_t np = F.n_passes();
         s->info.n_passes = np;
@@ -773,7 +772,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
             if (mb) std::memcpy(host.data() + ob, s->mats.data(), mb);
             SVB_TRY(wait_plan_buf(s));
             SVB_CUDA(grow(s->plan_buf, host.size()), "cudaMalloc(plan)");
-            SVB_CUDA(cudaMemcpyAsync(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice, s->own_stream),
+            SVB_CUDA(cudaMemcpyAsync(s->plan_buf.p, host.data(), host.size(), cudaMemcpyHostToDevice, nullptr),
                      "plan upload");
             s->small_ops = static_cast<const SmallOp*>(s->plan_buf.p);
             s->small_mats = reinterpret_cast<const double*>(static_cast<unsigned char*>(s->plan_buf.p) + ob);
@@ -784,7 +783,7 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
     }
     // sweeps of single gates have their matrices in the launches
     s->uploading = engine != SVB_ENGINE_PER_GATE || s->small_ops;
-    if (s->uploading) SVB_CUDA(cudaEventRecord(s->uploaded, s->own_stream), "cudaEventRecord");
+    if (s->uploading) SVB_CUDA(cudaEventRecord(s->uploaded, nullptr), "cudaEventRecord");
     s->have_circuit = true;
     return SVB_OK;
 }
@@ -830,11 +829,13 @@ svb_status svb_run(svb_sim* s, void* stream)
     }
     if (use_graph(s)) {
         if (!s->graph) {
-            SVB_CUDA(cudaStreamBeginCapture(s->own_stream, cudaStreamCaptureModeThreadLocal),
+            if (!s->capture_stream)
+                SVB_CUDA(cudaStreamCreateWithFlags(&s->capture_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+            SVB_CUDA(cudaStreamBeginCapture(s->capture_stream, cudaStreamCaptureModeThreadLocal),
                      "cudaStreamBeginCapture");
-            svb_status rc = launch_all(s, s->own_stream);
+            svb_status rc = launch_all(s, s->capture_stream);
             cudaGraph_t g = nullptr;
-            cudaError_t e = cudaStreamEndCapture(s->own_stream, &g);
+            cudaError_t e = cudaStreamEndCapture(s->capture_stream, &g);
             if (rc != SVB_OK) { if (g) cudaGraphDestroy(g); return rc; }
             if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
             e = cudaGraphInstantiate(&s->graph, g, 0);

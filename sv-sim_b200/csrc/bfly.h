@@ -142,9 +142,9 @@ bool plan_bfly(const std::vector<EOp>& ops, int n, int precision, BfPlan& plan, 
 
 // The coefficients as the kernel of FP32 states reads them.
 std::vector<float> bfly_coefs32(const BfPlan& plan);
-// The plan in one device buffer, copied from the host on stream s; `buf` grows as needed and no
-// kernel may still be reading it.
-cudaError_t upload_bfly(const BfPlan& plan, int precision, GrowBuf& buf, DevBfBuffers& dev, cudaStream_t s);
+// The plan in one device buffer, copied from the host on the default stream (it may return before
+// the copy has arrived); `buf` grows as needed and no kernel may still be reading it.
+cudaError_t upload_bfly(const BfPlan& plan, int precision, GrowBuf& buf, DevBfBuffers& dev);
 // one pass over the state
 template <typename T>
 cudaError_t launch_bfly_pass(void* state, int n, int pass_index, const DevBfBuffers& b, cudaStream_t s);

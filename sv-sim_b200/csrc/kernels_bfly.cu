@@ -172,7 +172,7 @@ k_bfly(typename BfWord<T>::type* __restrict__ sv, const BfPass* __restrict__ pas
 
 }  // namespace
 
-cudaError_t upload_bfly(const BfPlan& plan, int precision, GrowBuf& buf, DevBfBuffers& dev, cudaStream_t s)
+cudaError_t upload_bfly(const BfPlan& plan, int precision, GrowBuf& buf, DevBfBuffers& dev)
 {
     const bool fp32 = precision == SVB_FP32;
     // BfOp is read in 16-byte words: the passes' part is rounded up
@@ -190,7 +190,7 @@ cudaError_t upload_bfly(const BfPlan& plan, int precision, GrowBuf& buf, DevBfBu
         std::memcpy(h + sp + so + sr, plan.coefs.data(), sc);
     }
     cudaError_t e = grow(buf, host.size());
-    if (e == cudaSuccess && !host.empty()) e = cudaMemcpyAsync(buf.p, h, host.size(), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && !host.empty()) e = cudaMemcpyAsync(buf.p, h, host.size(), cudaMemcpyHostToDevice, nullptr);
     unsigned char* d = static_cast<unsigned char*>(buf.p);
     dev.passes = reinterpret_cast<BfPass*>(d);
     dev.ops = reinterpret_cast<BfOp*>(d + sp);

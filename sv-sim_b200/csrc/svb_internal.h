@@ -548,7 +548,7 @@ struct Sim {
     const double* small_mats = nullptr;
     bool have_circuit = false;
     cudaGraphExec_t graph = nullptr;
-    cudaStream_t own_stream = nullptr;    // uploads of plans and capture of their graphs
+    cudaStream_t capture_stream = nullptr;
     cudaEvent_t uploaded = nullptr;       // behind the plan's copies
     bool uploading = false;               // not yet seen to be complete
     svb_plan_info info{};
