@@ -672,13 +672,13 @@ svb_status set_circuit_lowered(Sim* s, std::vector<EOp>& eops, const svb_gate* g
         bool ok = false;
         if (compare) {
             try {
-                helper = std::thread([&] { ok = plan_bfly(s->eops, n, s->precision, B, true); });
+                helper = std::thread([&] { ok = plan_bfly(s->eops, n, s->precision, B); });
             } catch (const std::system_error&) {
             }
             pairs_planned = plan_pairs(s->eops, n, s->pairs, &s->mats);
         }
         if (helper.joinable()) helper.join();
-        else ok = plan_bfly(s->eops, n, s->precision, B, true);
+        else ok = plan_bfly(s->eops, n, s->precision, B);
         bfly = ok && (!pairs_planned || bfly_cheaper(B, s->pairs));
         if (bfly) s->pairs = PairPlan{};
         if (!bfly && s->engine_req == SVB_ENGINE_BUTTERFLY) {

@@ -250,7 +250,7 @@ struct PassPlanner {
     const int n;
     const int M;                         // local positions
     const int pack;                      // 1: position 0 is the half of a packed unit
-    const bool fp32, tune;
+    const bool fp32;
     M2* pend;                            // pending matrix of every qubit
     int local_q[BF_MAX_POS];
     int pos_of[64];
@@ -610,7 +610,7 @@ struct PassPlanner {
                 regs[k++] = p;
                 in |= 1u << p;
             }
-        if (!tune || (int)order.size() <= BF_RB || wanted < BF_RB) return;
+        if ((int)order.size() <= BF_RB || wanted < BF_RB) return;
         // one qubit at a time exchanged for a later one, where the stage gets more done; the
         // first need stays, so that every stage gets on
         auto value = [&](const int* r) {
@@ -966,7 +966,7 @@ std::vector<float> bfly_coefs32(const BfPlan& plan)
     return f;
 }
 
-bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, bool tune)
+bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan)
 {
     plan = BfPlan{};
     const bool fp32 = precision == SVB_FP32;
@@ -999,7 +999,7 @@ bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, 
             cuts.push_back({L, taken});
             return std::vector<int>{};
         },
-        tune ? 32 : 1);
+        32);
     // the next cut that touches each qubit, from the last one backwards
     std::vector<std::array<int32_t, 64>> next(cuts.size());
     {
@@ -1014,7 +1014,7 @@ bool plan_bfly(const std::vector<EOp>& raw, int n, int precision, BfPlan& plan, 
     }
     std::vector<M2> pend(64, ident2());
     uint8_t cls[64] = {0};
-    PassPlanner pp{plan, n, M, fp32 ? 1 : 0, fp32, tune, pend.data()};
+    PassPlanner pp{plan, n, M, fp32 ? 1 : 0, fp32, pend.data()};
     for (size_t ci = 0; ci < cuts.size(); ci++) {
         const uint64_t L = cuts[ci].first;
         std::vector<Item> ends;

@@ -135,10 +135,9 @@ enum class BfChoice { BLOCKS, BUTTERFLIES, COMPARE };
 BfChoice bfly_choice(const std::vector<EOp>& ops, int n, int precision);
 // the comparison of the FP64 plans of one circuit
 bool bfly_cheaper(const BfPlan& b, const PairPlan& p);
-// `tune` spends more host time on the choice of register qubits (1.5-3x the planning time).
 // False if a layout came out that the kernel cannot address, or a pass that does nothing of
 // what is left (neither has been seen; the caller then takes another engine).
-bool plan_bfly(const std::vector<EOp>& ops, int n, int precision, BfPlan& plan, bool tune);
+bool plan_bfly(const std::vector<EOp>& ops, int n, int precision, BfPlan& plan);
 
 // The coefficients as the kernel of FP32 states reads them.
 std::vector<float> bfly_coefs32(const BfPlan& plan);

@@ -760,7 +760,7 @@ int run_bfly(int n, const BfPlan& plan, std::vector<typename VecOf<T>::type>& sv
 
 // (re, im) <- circuit applied to (re, im).  stats: passes, gates, diagonal ops, register
 // moves, relayouts, eight-lane shared-memory phases with bank conflicts, all phases.
-extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, int precision, int tune, int execute,
+extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, int precision, int execute,
                             double* re, double* im, uint64_t* stats)
 {
     std::vector<EOp> eops;
@@ -768,7 +768,7 @@ extern "C" int emu_bfly_run(uint32_t n, const svb_gate* gates, size_t n_gates, i
         if (!lower_gate(gates[i], (int32_t)i, eops)) return -1;
     if (!bfly_supported(eops, (int)n, precision)) return -5;
     BfPlan plan;
-    if (!plan_bfly(eops, (int)n, precision, plan, tune != 0)) return -8;
+    if (!plan_bfly(eops, (int)n, precision, plan)) return -8;
     stats[0] = plan.passes.size();
     stats[1] = plan.n_gates2;
     stats[2] = plan.n_diags;
@@ -809,6 +809,6 @@ extern "C" int emu_bfly_choice(uint32_t n, const svb_gate* gates, size_t n_gates
     if (choice != BfChoice::COMPARE) return choice == BfChoice::BUTTERFLIES;
     BfPlan b;
     PairPlan p;
-    if (!plan_bfly(eops, (int)n, precision, b, true)) return 0;
+    if (!plan_bfly(eops, (int)n, precision, b)) return 0;
     return !plan_pairs(eops, (int)n, p) || bfly_cheaper(b, p);
 }

@@ -413,13 +413,13 @@ def phase_circuit(n, seed, reps=2):
     return G.to_array(gl)
 
 
-def run_bfly(lib, n, gates, precision, tune=1, seed=3):
+def run_bfly(lib, n, gates, precision, seed=3):
     rng = np.random.default_rng(seed)
     st = rng.standard_normal((2, 1 << n))
     st /= np.sqrt((st ** 2).sum())
     re, im = st[0].copy(), st[1].copy()
     stats = (ctypes.c_uint64 * 8)()
-    rc = lib.emu_bfly_run(n, gates.ctypes.data, ctypes.c_size_t(len(gates)), precision, tune, 1, re.ctypes.data_as(_dp),
+    rc = lib.emu_bfly_run(n, gates.ctypes.data, ctypes.c_size_t(len(gates)), precision, 1, re.ctypes.data_as(_dp),
                           im.ctypes.data_as(_dp), stats)
     return rc, (re, im), st, list(stats)
 
@@ -445,16 +445,13 @@ def test_butterfly_plan_from_random_states(emu, oracle, n, kind, precision):
     else:
         g = mixed_circuit(n, 2, seed=n)
         g = g[(g["op"] != G.OP["SRN"]) & (g["op"] != G.OP["R"])]
-    want = None
-    for tune in (0, 1):
-        rc, got, st, stats = run_bfly(emu, n, g, precision, tune)
-        assert rc == 0 and stats[0] >= 1
-        if want is None:
-            want = oracle.run(n, g, state=(st[0], st[1]))
-        err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
-        # 2-norm error: one rounding (eps / 2 of the norm at most) a gate, in quadrature, times 8
-        eps = 2.2e-16 if precision == 0 else 1.2e-7
-        assert err <= 8 * eps * np.sqrt(max(len(g), 100)), (tune, err)
+    rc, got, st, stats = run_bfly(emu, n, g, precision)
+    assert rc == 0 and stats[0] >= 1
+    want = oracle.run(n, g, state=(st[0], st[1]))
+    err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+    # 2-norm error: one rounding (eps / 2 of the norm at most) a gate, in quadrature, times 8
+    eps = 2.2e-16 if precision == 0 else 1.2e-7
+    assert err <= 8 * eps * np.sqrt(max(len(g), 100)), err
 
 
 def test_butterfly_plan_rejects_what_it_cannot_split(emu):
@@ -493,11 +490,10 @@ def test_butterfly_plan_packed_control_onto_a_shared_register(emu, oracle, n, t,
     register: a row beside the packed one that differs between the halves of a unit has no
     address.  FP32 rounding only (the circuits move amplitudes and negate them)."""
     g = shared_register(n, t, y, phases)
-    for tune in (0, 1):
-        rc, got, st, _ = run_bfly(emu, n, g, 1, tune)
-        want = oracle.run(n, g, state=(st[0], st[1]))
-        err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
-        assert rc == 0 and err <= 1.2e-7
+    rc, got, st, _ = run_bfly(emu, n, g, 1)
+    want = oracle.run(n, g, state=(st[0], st[1]))
+    err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
+    assert rc == 0 and err <= 1.2e-7
 
 
 def short_circuit(n, rng):
@@ -525,7 +521,7 @@ def test_butterfly_plan_on_random_short_circuits(emu, oracle, precision):
         rng = np.random.default_rng(seed)
         n = int(rng.integers(12, 15)) + precision
         g = short_circuit(n, rng)
-        rc, got, st, _ = run_bfly(emu, n, g, precision, tune=seed & 1, seed=seed)
+        rc, got, st, _ = run_bfly(emu, n, g, precision, seed)
         want = oracle.run(n, g, state=(st[0], st[1]))
         err = np.sqrt(np.sum((got[0] - want[0]) ** 2 + (got[1] - want[1]) ** 2))
         assert rc == 0 and err <= 8 * eps * np.sqrt(100), (seed, rc, err)
@@ -541,7 +537,7 @@ def test_butterfly_plan_of_a_circuit_with_many_cuts(emu):
     for reps in (100, 200, 31000):
         g = np.tile(one, reps)
         st = (ctypes.c_uint64 * 8)()
-        assert emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), 0, 0, 0, None, None, st) == 0
+        assert emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), 0, 0, None, None, st) == 0
         stats[reps] = np.array([int(x) for x in st])
     period = stats[200] - stats[100]
     assert stats[31000][0] > 32767
@@ -562,7 +558,7 @@ def test_butterfly_plan_keeps_large_amplitudes_finite(emu, oracle, precision, fa
     st /= np.sqrt(np.max(st[0] ** 2 + st[1] ** 2))
     re, im = st[0] * factor, st[1] * factor
     stats = (ctypes.c_uint64 * 8)()
-    rc = emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), precision, 1, 1,
+    rc = emu.emu_bfly_run(n, ctypes.c_void_p(g.ctypes.data), ctypes.c_size_t(len(g)), precision, 1,
                           re.ctypes.data_as(_dp), im.ctypes.data_as(_dp), stats)
     want = oracle.run(n, g, state=(st[0], st[1]))
     err = np.sqrt(np.sum((re / factor - want[0]) ** 2 + (im / factor - want[1]) ** 2))
