@@ -55,7 +55,7 @@ def parse():
     ap.add_argument("--qubits", type=int, default=N_QUBITS,
                     help="state size (smaller cases are for profiling only)")
     ap.add_argument("--tile-bits", type=int, default=12)
-    ap.add_argument("--engine", choices=["auto", "pairs", "staged"], default="auto",
+    ap.add_argument("--engine", choices=["auto", "butterfly", "pairs", "staged"], default="auto",
                     help="FP64 engine of the headline step")
     ap.add_argument("--form", choices=["headline", "pergate", "fused", "qaoa", "capacity", "adjoint", "density",
                                        "config1", "tuning", "batch", "refgpu"],
@@ -311,8 +311,8 @@ def run_ours(args):
     n_gates = len(circuit)
 
     h = nat.Handle(nq, device, nat.SVB_FP64)
-    h.set_engine({"auto": nat.ENGINE_AUTO, "pairs": nat.ENGINE_PAIRS, "staged": nat.ENGINE_STAGED}[args.engine],
-                 args.tile_bits if args.engine == "staged" else 0, 0)
+    h.set_engine({"auto": nat.ENGINE_AUTO, "butterfly": nat.ENGINE_BUTTERFLY, "pairs": nat.ENGINE_PAIRS,
+                  "staged": nat.ENGINE_STAGED}[args.engine], args.tile_bits if args.engine == "staged" else 0, 0)
     h.set_circuit(circuit)
     info = h.plan_info()
     stream = torch.cuda.current_stream(device)
@@ -356,8 +356,8 @@ def run_ours(args):
     # AUTO's choice without tensor-core blocks: butterflies
     pairs = args.engine != "staged"
     butterflies = pairs and int(info.n_blocks) == 0
-    tfile = os.path.join(ROOT, "profiles", "pairs_fp64_traffic.txt" if pairs else "staged_fp64_traffic.txt")
-    if os.path.exists(tfile) and not butterflies:
+    tfile = os.path.join(ROOT, "profiles", ("bfly" if butterflies else "pairs" if pairs else "staged") + "_fp64_traffic.txt")
+    if os.path.exists(tfile):
         for ln in open(tfile):
             if ln.startswith("bytes_per_launch_n30"):
                 traffic = float(ln.split("=")[1])

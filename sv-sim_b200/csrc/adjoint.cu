@@ -247,7 +247,9 @@ enum { AS_LOC_REG = 0, AS_LOC_THREAD = 1, AS_LOC_TILE = 2 };
 // amplitude, and no need for the pair: a differentiated RZ stays a diagonal op that may sit
 // on any qubit).  Forming dU psi by a general 2x2 took 24, and undoing a real or diagonal
 // gate by a general 2x2 twice the multiply-adds: the FP64 pipe was the largest part of the
-// sweep (n = 20 ansatz: a gradient 4.89 ms, now 3.42).
+// sweep (n = 20 ansatz: a gradient 4.89 ms, now 3.42).  Four CTAs an SM need 128 registers a
+// thread, which spills 56 bytes; the FP64 pipe is 9-16% busy, the latency of loads and barriers
+// in tiles of 1,024 amplitudes is what is left.
 struct AdjStageOp {
     uint8_t kind;      // AT_C1, AT_DIAG, AT_CX, AT_REAL
     uint8_t j;         // C1 / CX: register bit of the target; DIAG: bit of the qubit in its location

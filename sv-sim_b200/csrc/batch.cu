@@ -384,8 +384,9 @@ __global__ void __launch_bounds__(QB_THREADS, 1) k_qaoa(QaoaArgs A)
             // stages 0..3: mixer on the owned bits, with exchanges between stages
             // A pass whose bits from jb on begin above a stage's has nothing to do there and
             // goes to the next owner at once: the exchange it spares costs more than the
-            // branch (problems of 10 to 22 qubits, 4 layers, with gradients: 192 in FP64
-            // 34.69 -> 34.32 ms, 512 in FP32 63.30 -> 61.88 ms).
+            // branch (problems of 10 to 22 qubits, 4 layers, with gradients, both ways in turn:
+            // 192 in FP64 38.12 -> 37.75 ms, 512 in FP32 63.49 -> 62.08 ms; runs of one side
+            // differ by 0.1%).
             constexpr int own2 = C::reg_bit(2, 0), own3 = C::reg_bit(3, 0);
             if (fwd) {
                 // the exchanges alternate between the two buffers (lambda's is free on the

@@ -8,7 +8,9 @@
 // slots, so every other instruction adds to them), a redistribution 1,500 cycles, tile loads
 // and stores 58 ms.  The two CTAs of an SM overlap these little; handing the right to compute
 // from one to the other made it 242 ms, prefetching the next tile into L2 and starting half
-// of the CTAs later changed nothing, loading tiles without cp.async made it 259 ms.
+// of the CTAs later changed nothing, loading tiles without cp.async made it 259 ms.  So neither
+// memory nor the FP64 pipe is full: 25% of the DRAM rate and 35% of the pipe's in a pass at 26
+// qubits.  Registers: 128, the most that two CTAs leave; <float> spills 128 bytes a thread.
 #include <cstring>
 #include <vector>
 

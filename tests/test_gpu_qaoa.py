@@ -157,9 +157,9 @@ def test_sharded_wrapper_single_process_equals_batch():
 
 @pytest.mark.parametrize("precision", [0, 1])
 def test_mixer_angles_over_the_whole_circle(precision):
-    """beta where cos or sin vanish, at the line between the two forms of the mixer (pi / 4),
-    negative and beyond pi, at sizes on both sides of every line of the pass structure (one
-    tile; high passes that own 1 to 10 bits): energies and gradients against svb_adjoint."""
+    """beta where cos(beta) or sin(beta) vanish or nearly do, where they are equal, negative and
+    beyond pi, at sizes on both sides of every line of the pass structure (one tile; high passes
+    that own 1 to 10 bits): energies and gradients against svb_adjoint."""
     from svsim_b200 import _native as nat
     rng = np.random.default_rng(8)
     betas = [0.0, np.pi / 2, np.pi / 4, 3 * np.pi / 4, np.pi, -0.3, 1e-9, np.pi / 2 - 1e-9, 2.0, np.pi / 4 + 1e-12]
