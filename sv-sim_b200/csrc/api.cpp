@@ -99,6 +99,8 @@ void free_scratch(Sim* s)
 {
     free_adjoint_scratch(s->adj);
     release(s->plan_buf);
+    for (GrowBuf& b : s->captured_bufs) release(b);
+    s->captured_bufs.clear();
     cudaFree(s->mscr.cdf);
     cudaFree(s->mscr.uniforms);
     cudaFree(s->mscr.samples);
@@ -557,11 +559,15 @@ svb_status mark_plan_buf(Sim* s, cudaStream_t st, bool capturing)
 }
 
 // Before plan_buf is written again: waits for the runs that read it, and for no other
-// handle's work.
+// handle's work.  A buffer that a caller's graph reads stays as it is until the handle goes.
 svb_status wait_plan_buf(Sim* s)
 {
-    if (s->plan_reader == Sim::READ) SVB_CUDA(cudaEventSynchronize(s->plan_read), "kernel execution");
-    else if (s->plan_reader == Sim::CAPTURED) SVB_CUDA(cudaDeviceSynchronize(), "kernel execution");
+    if (s->plan_reader == Sim::READ) {
+        SVB_CUDA(cudaEventSynchronize(s->plan_read), "kernel execution");
+    } else if (s->plan_reader == Sim::CAPTURED) {
+        s->captured_bufs.push_back(s->plan_buf);
+        s->plan_buf = GrowBuf{};
+    }
     s->plan_reader = Sim::UNREAD;
     return SVB_OK;
 }

@@ -544,6 +544,7 @@ struct Sim {
                                    // circuit to circuit
     enum { UNREAD, READ, CAPTURED } plan_reader = UNREAD;    // runs that read plan_buf
     cudaEvent_t plan_read = nullptr;      // READ: behind the last of them
+    std::vector<GrowBuf> captured_bufs;   // earlier ones that callers' graphs read
     const SmallOp* small_ops = nullptr;   // per-gate engine on a small state: into plan_buf
     const double* small_mats = nullptr;
     bool have_circuit = false;

@@ -139,3 +139,28 @@ def test_pauli_sums_on_both_sides_of_the_lines_between_their_forms(oracle, n, co
         binding["idx"] = -1
         ea, _ = h.adjoint(g, binding, 0, t)
         assert abs(ea - want) <= bound
+
+
+def test_a_captured_run_keeps_its_circuit(oracle):
+    """A graph that holds a run replays that circuit after the handle has others (of as many
+    gates, so that any of the lists is one that the launch can read)."""
+    import torch
+    from svsim_b200 import _native as nat
+    n = 8
+    a, b, c = (circuits.random_matching_circuit(n, 6, seed=s) for s in range(3))
+    h = nat.Handle(n, 0, nat.SVB_FP64)
+    h.set_engine(nat.ENGINE_PER_GATE)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    h.set_circuit(a)
+    with torch.cuda.graph(graph, stream=side):
+        h.run(side.cuda_stream)
+    for g in (b, c):
+        h.set_circuit(g)
+        h.run(side.cuda_stream)
+    with torch.cuda.stream(side):
+        graph.replay()
+    h.run(side.cuda_stream)
+    side.synchronize()
+    re, im = h.get_state()
+    want = oracle.run(n, np.concatenate([b, c, a, c]))
+    assert np.array_equal(re, want[0]) and np.array_equal(im, want[1])
