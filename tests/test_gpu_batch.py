@@ -163,3 +163,25 @@ def test_pair_engine_request_on_fp32_and_small_circuits(oracle):
     re, im = oracle.run(13, srn[0][1])
     assert np.max(np.abs(b.state(0) - (re + 1j * im))) <= 1e-12
     b.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_new_angles_for_circuits_of_both_engines(oracle, precision):
+    """A batch of 8- and 14-qubit circuits, of which the pair engine runs the larger ones (FP64),
+    with new angles twice: states and energies of the new angles, energies one product a term and
+    amplitude from the oracle's."""
+    nat = native()
+    pcs = [circuits.hardware_efficient_ansatz(n, 3, seed=n + i) for i, n in enumerate((8, 14, 14, 8, 11))]
+    terms = [circuits.zz_x_hamiltonian(pc.n) for pc in pcs]
+    b = nat.CircuitBatch([(pc.n, pc.gates) for pc in pcs], terms, precision=precision)
+    rng = np.random.default_rng(5)
+    tol = 1e-12 if precision == 0 else 1e-4
+    for _ in range(2):
+        gates = [pc.evaluated(rng.uniform(-np.pi, np.pi, len(pc.params))) for pc in pcs]
+        e = b.run(np.concatenate(gates))
+        for i, (pc, g) in enumerate(zip(pcs, gates)):
+            want = oracle.run(pc.n, g)
+            st = b.state(i)
+            assert np.max(np.abs(st.real - want[0])) < tol and np.max(np.abs(st.imag - want[1])) < tol
+            assert abs(e[i] - oracle.expectation(pc.n, *want, terms[i])) < 10 * tol
+    b.close()
